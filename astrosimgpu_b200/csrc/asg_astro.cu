@@ -108,7 +108,7 @@ __device__ __forceinline__ void advance_cell(const StepArgs& a, const AstroArray
 // and two interleaved RK4 chains); kMinBlocks sets the register budget
 // through __launch_bounds__ (65536 / (kBlock * kMinBlocks) per thread).
 template <bool kUniform, int kInput, bool kNoise, int kCells, int kBlock, int kMinBlocks>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(StepArgs a, AstroArrays s) {
+__global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __grid_constant__ StepArgs a, AstroArrays s) {
     const std::int64_t step =
         (kInput == kInputBernoulli) ? (*a.step_base + a.step_offset) : 0;
     const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
@@ -347,6 +347,7 @@ AstroK make_astro_k(const double* c, double h_step, int substeps) {
     k.h = h_step;
     k.h6 = h_step / 6.0;
     k.substeps = substeps;
+    k.ieee = astro_needs_ieee(k);
     return k;
 }
 

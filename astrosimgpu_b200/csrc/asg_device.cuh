@@ -196,6 +196,60 @@ __host__ __device__ __forceinline__ bool diff_param_ok(double p) {
     return m >= 0x1p-906 && m <= 0x1p976;
 }
 
+// a / b for a divisor computed on the fly, from a seed y0 of 1/b (relative
+// error at most 2^-19): two Newton steps y <- y + y (1 - b y) leave y within
+// (1/2 + 2^-22) ulp of 1/b, and Markstein's correction (see div_by) of
+// q = RN(a y) gives the IEEE quotient.  Seven FP64 operations and no branch,
+// so the four divisions of a Li-Rinzel right-hand side interleave; the
+// compiler's division takes eight and a slow-path test each.
+//
+// The correction is exact although y need not be the correctly rounded
+// reciprocal.  With b scaled into [1, 2), q off by r/b and a midpoint m of
+// two doubles next to a/b, the last sum errs by |r| |y - 1/b|, which must
+// stay below |a/b - m| >= 2^-105 / b (a - b m is a non-zero multiple of
+// 2^-105).  That holds when b^2 (1 + 2^-22) < 4: for every b whose top 20
+// fraction bits are not all ones.  Those divisors (div_newton_excluded, one
+// in 2^20) and operands outside the exponent range [2^-400, 2^400] are the
+// caller's to divide with the IEEE division.
+// tests/div_newton_check.cu compares it with IEEE division, for seeds of any
+// error up to the bound.
+__host__ __device__ __forceinline__ double div_newton(double a, double b, double y0) {
+    const double e0 = fma(-b, y0, 1.0);
+    const double y1 = fma(y0, e0, y0);
+    const double e1 = fma(-b, y1, 1.0);
+    const double y = fma(y1, e1, y1);
+    const double q = a * y;
+    const double r = fma(-b, q, a);
+    return fma(r, y, q);
+}
+
+__host__ __device__ __forceinline__ unsigned high_word(double a) {
+#ifdef __CUDA_ARCH__
+    return static_cast<unsigned>(__double2hiint(a));
+#else
+    std::uint64_t u;
+    __builtin_memcpy(&u, &a, sizeof u);
+    return static_cast<unsigned>(u >> 32);
+#endif
+}
+
+__host__ __device__ __forceinline__ unsigned div_newton_excluded(double b) {
+    return (~high_word(b) & 0xFFFFFu) == 0u ? 1u : 0u;
+}
+
+// Not a positive number in [2^-100, 2^101): zero, negative, tiny, huge, NaN.
+__host__ __device__ __forceinline__ unsigned not_moderate(double a) {
+    return high_word(a) - (923u << 20) >= (201u << 20) ? 1u : 0u;
+}
+
+// The seed: the hardware's approximate reciprocal (the PTX instruction reads
+// and writes the upper 32 bits of its operand and result: about 20 bits).
+__device__ __forceinline__ double rcp_seed(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+}
+
 // ------------------------------------------------------ Li-Rinzel astrocyte
 
 // Population constants, with the run-time constant products of the
@@ -212,33 +266,50 @@ struct AstroK {
     double h;       // h_step
     double h6;      // h_step / 6.0
     int substeps;
+    unsigned ieee;  // a constant outside div_newton's range: divide in IEEE only
 };
+
+// Whether the constants keep the operands of the right-hand side's four
+// divisions within div_newton's range for every moderate Ca and IP3.
+__host__ inline unsigned astro_needs_ieee(const AstroK& k) {
+    return not_moderate(k.Kd_IP3_1) | not_moderate(k.Kd_IP3_2) | not_moderate(k.Kd_act) |
+           not_moderate(k.serca) | not_moderate(k.km2) | not_moderate(k.ah);
+}
 
 struct AstroRates {
     double Ca, IP3, h;
 };
 
-// d/dt of (Ca, IP3, h) for one cell.
+// d/dt of (Ca, IP3, h) for one cell, the four divisions by state-dependent
+// divisors through div_newton (`bad` collects what that must not divide) or,
+// with kIeee, as IEEE divisions.
 // `tau` and `inv_tau` (its correctly rounded reciprocal) give dIP3 with
 // div_diff_by; the result is the IEEE quotient (IP3_0 - IP3) / tau, as the ER
 // calcium is (Ca_tot - Ca) / ratio_ER_cyt, for Ca_tot and IP3_0 within
 // diff_param_ok (checked where the parameters enter the engine).
-__device__ __forceinline__ AstroRates li_rinzel(const AstroK& k, double ca_tot, double ip3_0,
-                                                double tau, double inv_tau, double ca, double ip3,
-                                                double hh, double noise) {
+template <bool kIeee>
+__device__ __forceinline__ AstroRates li_rinzel_rates(const AstroK& k, double ca_tot,
+                                                      double ip3_0, double tau, double inv_tau,
+                                                      double ca, double ip3, double hh,
+                                                      double noise, unsigned& bad) {
+    auto div = [&bad](double a, double b) {
+        if (kIeee) return a / b;
+        bad |= div_newton_excluded(b);
+        return div_newton(a, b, rcp_seed(b));
+    };
     const double er = div_diff_by(ca_tot, ca, k.ratio_ER_cyt, k.inv_ratio);  // ER calcium
     const double ip3_k1 = ip3 + k.Kd_IP3_1;
-    const double m = ip3 / ip3_k1;                      // IP3 activation
-    const double n = ca / (ca + k.Kd_act);              // Ca activation
+    const double m = div(ip3, ip3_k1);            // IP3 activation
+    const double n = div(ca, ca + k.Kd_act);      // Ca activation
     const double m3 = m * m * m;
     const double n3 = n * n * n;
     const double h3 = hh * hh * hh;
     const double gradient = er - ca;
     const double release = k.chan * m3 * n3 * h3 * gradient;
     const double ca2 = ca * ca;
-    const double uptake = k.serca * ca * ca / (k.km2 + ca2);
+    const double uptake = div(k.serca * ca * ca, k.km2 + ca2);
     const double leak = k.leak * gradient;
-    const double open_rate = k.ah * ip3_k1 / (ip3 + k.Kd_IP3_2);
+    const double open_rate = div(k.ah * ip3_k1, ip3 + k.Kd_IP3_2);
     const double close_rate = k.k_IP3R * ca;
     AstroRates r;
     r.Ca = release - uptake + leak + noise;
@@ -247,12 +318,40 @@ __device__ __forceinline__ AstroRates li_rinzel(const AstroK& k, double ca_tot, 
     return r;
 }
 
+__device__ __forceinline__ AstroRates li_rinzel_rates_ieee(const AstroK& k, double ca_tot,
+                                                           double ip3_0, double tau,
+                                                           double inv_tau, double ca, double ip3,
+                                                           double hh, double noise) {
+    unsigned unused = 0u;
+    return li_rinzel_rates<true>(k, ca_tot, ip3_0, tau, inv_tau, ca, ip3, hh, noise, unused);
+}
+
+// Out of line: the rare evaluation (a zero, negative or extreme Ca or IP3, an
+// excluded divisor) redone with IEEE divisions.
+static __device__ __noinline__ AstroRates li_rinzel_ieee(const AstroK& k, double ca_tot,
+                                                         double ip3_0, double tau,
+                                                         double inv_tau, double ca, double ip3,
+                                                         double hh, double noise) {
+    return li_rinzel_rates_ieee(k, ca_tot, ip3_0, tau, inv_tau, ca, ip3, hh, noise);
+}
+
+__device__ __forceinline__ AstroRates li_rinzel(const AstroK& k, double ca_tot, double ip3_0,
+                                                double tau, double inv_tau, double ca, double ip3,
+                                                double hh, double noise) {
+    unsigned bad = k.ieee | not_moderate(ca) | not_moderate(ip3);
+    AstroRates r = li_rinzel_rates<false>(k, ca_tot, ip3_0, tau, inv_tau, ca, ip3, hh, noise, bad);
+    if (bad != 0u) r = li_rinzel_ieee(k, ca_tot, ip3_0, tau, inv_tau, ca, ip3, hh, noise);
+    return r;
+}
+
 // Input jump, then `substeps` classical RK4 steps with the physical clamps.
 // kUnroll = false runs the four stages as a loop (one copy of the right-hand
 // side in the instruction stream, for kernels that also hold other roles'
 // code); the weighted stage sum is accumulated left to right either way, so
 // both forms perform the same IEEE operations in the same order.
-template <bool kUnroll = true>
+// kNewton = false divides with the compiler's IEEE division (the network step
+// kernels, whose other roles it slows: use_case 3.43 -> 3.63 us per step).
+template <bool kUnroll = true, bool kNewton = true>
 __device__ __forceinline__ void astro_rk4(const AstroK& k, double ca_tot, double ip3_0, double tau,
                                           double inv_tau, double delta, double input, double noise,
                                           double& ca, double& ip3, double& hh) {
@@ -262,7 +361,9 @@ __device__ __forceinline__ void astro_rk4(const AstroK& k, double ca_tot, double
         double xCa = ca, xIP3 = ip3, xh = hh;     // stage inputs
 #pragma unroll(kUnroll ? 4 : 1)
         for (int st = 0; st < 4; ++st) {
-            const AstroRates r = li_rinzel(k, ca_tot, ip3_0, tau, inv_tau, xCa, xIP3, xh, noise);
+            const AstroRates r =
+                kNewton ? li_rinzel(k, ca_tot, ip3_0, tau, inv_tau, xCa, xIP3, xh, noise)
+                        : li_rinzel_rates_ieee(k, ca_tot, ip3_0, tau, inv_tau, xCa, xIP3, xh, noise);
             if (st == 0) {
                 sCa = r.Ca;
                 sIP3 = r.IP3;

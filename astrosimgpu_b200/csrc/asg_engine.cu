@@ -71,6 +71,7 @@ AstroK make_astro_k(const asg_astro_params& a, double h, int substeps) {
     k.h = h;
     k.h6 = h / 6.0;
     k.substeps = substeps;
+    k.ieee = astro_needs_ieee(k);
     return k;
 }
 

@@ -1107,7 +1107,7 @@ __device__ void astro_role(const InstDev& I, const StepInfo& S, const Work& wk) 
     if constexpr (kF32)
         astro_update_f32(I, ca_tot, ip3_0, tau, delta, ip3_in, noise, ca, ip3, hh);
     else
-        astro_rk4<false>(I.ak, ca_tot, ip3_0, tau, inv_tau, delta, ip3_in, noise, ca, ip3, hh);
+        astro_rk4<false, false>(I.ak, ca_tot, ip3_0, tau, inv_tau, delta, ip3_in, noise, ca, ip3, hh);
     I.Ca[a] = ca;
     I.IP3[a] = ip3;
     I.h[a] = hh;
