@@ -4,11 +4,9 @@
 // device.
 //
 // Layout: SoA FP64 arrays Ca, IP3, h (+ Ca_tot, IP3_0, tau_IP3, delta_IP3
-// when per-cell), 256-byte aligned.  Each thread owns two adjacent cells so
-// every state array is read and written with one coalesced 128-bit access
-// per thread, and the two independent RK4 chains interleave to cover FP64
-// latency.  Grid-stride loop over cell pairs; grid sized in multiples of
-// the SM count.
+// when per-cell), 256-byte aligned.  A thread owns one, two or four adjacent
+// cells (the launch shape), read and written with coalesced accesses; one
+// thread per unit of cells, no loop over the grid.
 //
 // Compiled with -fmad=false: results are bitwise equal to the host's
 // astro_advance (no transcendental on this path when noise is off).
@@ -69,8 +67,8 @@ struct StepArgs {
     std::uint64_t seed;
     double p, weight;
     std::uint64_t p_threshold;
-    const std::int64_t* step_base;  // device counter: step = *step_base + step_offset
-    int step_offset;
+    std::int64_t step0;  // the launch advances every cell by steps step0 .. step0 + n_steps - 1
+    int n_steps;
     std::int64_t i0;  // global index of the first cell of this launch (RNG streams)
 };
 
@@ -107,11 +105,17 @@ __device__ __forceinline__ void advance_cell(const StepArgs& a, const AstroArray
 // kCells adjacent cells per thread (1: 64-bit accesses, 2: 128-bit accesses
 // and two interleaved RK4 chains); kMinBlocks sets the register budget
 // through __launch_bounds__ (65536 / (kBlock * kMinBlocks) per thread).
+//
+// The Bernoulli workload needs nothing from outside between steps, so one
+// launch advances its cells by all of a call's steps with the state in
+// registers.  A launch per step spent the small sizes on launch latency and
+// the large ones on the state's round trip: per step 2.9 -> 0.68 us at 4,099
+// cells, 8.7 -> 6.1 us at 300,007, 213 -> 195 us at 10^7 (297 FP64
+// instructions per cell-step, 82 % of the FP64 pipe's rate: what bounds it).
 template <bool kUniform, int kInput, bool kNoise, int kCells, int kBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __grid_constant__ StepArgs a, AstroArrays s) {
-    const std::int64_t step =
-        (kInput == kInputBernoulli) ? (*a.step_base + a.step_offset) : 0;
-    const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
+    const int n_steps = kInput == kInputBernoulli ? a.n_steps : 1;
+    const std::int64_t u = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (kCells == 4) {
         // Four adjacent cells per thread (two 128-bit accesses per array):
         // four independent RK4 chains to interleave.
@@ -119,15 +123,17 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __
         double2* Ca2 = reinterpret_cast<double2*>(s.Ca);
         double2* IP32 = reinterpret_cast<double2*>(s.IP3);
         double2* h2 = reinterpret_cast<double2*>(s.h);
-        for (std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-             q < quads; q += stride) {
+        if (const std::int64_t q = u; q < quads) {
             double2 ca0 = Ca2[2 * q], ip30 = IP32[2 * q], hh0 = h2[2 * q];
             double2 ca1 = Ca2[2 * q + 1], ip31 = IP32[2 * q + 1], hh1 = h2[2 * q + 1];
             const std::int64_t i = 4 * q;
-            advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca0.x, ip30.x, hh0.x);
-            advance_cell<kUniform, kInput, kNoise>(a, s, i + 1, step, ca0.y, ip30.y, hh0.y);
-            advance_cell<kUniform, kInput, kNoise>(a, s, i + 2, step, ca1.x, ip31.x, hh1.x);
-            advance_cell<kUniform, kInput, kNoise>(a, s, i + 3, step, ca1.y, ip31.y, hh1.y);
+            for (int t = 0; t < n_steps; ++t) {
+                const std::int64_t step = a.step0 + t;
+                advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca0.x, ip30.x, hh0.x);
+                advance_cell<kUniform, kInput, kNoise>(a, s, i + 1, step, ca0.y, ip30.y, hh0.y);
+                advance_cell<kUniform, kInput, kNoise>(a, s, i + 2, step, ca1.x, ip31.x, hh1.x);
+                advance_cell<kUniform, kInput, kNoise>(a, s, i + 3, step, ca1.y, ip31.y, hh1.y);
+            }
             Ca2[2 * q] = ca0;
             IP32[2 * q] = ip30;
             h2[2 * q] = hh0;
@@ -143,7 +149,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __
         if (blockIdx.x == 0 && threadIdx.x < static_cast<unsigned>(a.n & 3)) {
             const std::int64_t i = 4 * quads + threadIdx.x;
             double ca = s.Ca[i], ip3 = s.IP3[i], hh = s.h[i];
-            advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca, ip3, hh);
+            for (int t = 0; t < n_steps; ++t)
+                advance_cell<kUniform, kInput, kNoise>(a, s, i, a.step0 + t, ca, ip3, hh);
             s.Ca[i] = ca;
             s.IP3[i] = ip3;
             s.h[i] = hh;
@@ -154,12 +161,14 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __
         double2* Ca2 = reinterpret_cast<double2*>(s.Ca);
         double2* IP32 = reinterpret_cast<double2*>(s.IP3);
         double2* h2 = reinterpret_cast<double2*>(s.h);
-        for (std::int64_t p = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-             p < pairs; p += stride) {
+        if (const std::int64_t p = u; p < pairs) {
             double2 ca = Ca2[p], ip3 = IP32[p], hh = h2[p];
             const std::int64_t i = 2 * p;
-            advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca.x, ip3.x, hh.x);
-            advance_cell<kUniform, kInput, kNoise>(a, s, i + 1, step, ca.y, ip3.y, hh.y);
+            for (int t = 0; t < n_steps; ++t) {
+                advance_cell<kUniform, kInput, kNoise>(a, s, i, a.step0 + t, ca.x, ip3.x, hh.x);
+                advance_cell<kUniform, kInput, kNoise>(a, s, i + 1, a.step0 + t, ca.y, ip3.y,
+                                                       hh.y);
+            }
             Ca2[p] = ca;
             IP32[p] = ip3;
             h2[p] = hh;
@@ -170,17 +179,18 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) astro_step_kernel(const __
         if ((a.n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
             const std::int64_t i = a.n - 1;
             double ca = s.Ca[i], ip3 = s.IP3[i], hh = s.h[i];
-            advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca, ip3, hh);
+            for (int t = 0; t < n_steps; ++t)
+                advance_cell<kUniform, kInput, kNoise>(a, s, i, a.step0 + t, ca, ip3, hh);
             s.Ca[i] = ca;
             s.IP3[i] = ip3;
             s.h[i] = hh;
             if (kInput == kInputArrayZero) s.input[i] = 0.0;
         }
     } else {
-        for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-             i < a.n; i += stride) {
+        if (const std::int64_t i = u; i < a.n) {
             double ca = s.Ca[i], ip3 = s.IP3[i], hh = s.h[i];
-            advance_cell<kUniform, kInput, kNoise>(a, s, i, step, ca, ip3, hh);
+            for (int t = 0; t < n_steps; ++t)
+                advance_cell<kUniform, kInput, kNoise>(a, s, i, a.step0 + t, ca, ip3, hh);
             s.Ca[i] = ca;
             s.IP3[i] = ip3;
             s.h[i] = hh;
@@ -199,15 +209,18 @@ constexpr Shape kShapes[] = {{2, 128, 4}, {1, 128, 8}, {1, 256, 4}, {2, 128, 6},
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
 template <bool kUniform, int kInput, bool kNoise>
-cudaError_t launch_astro(int shape, int sms, StepArgs a, AstroArrays s, cudaStream_t st) {
+cudaError_t launch_astro(int shape, StepArgs a, AstroArrays s, cudaStream_t st) {
     // Independent noise (log and cos per cell) is compiled for one shape: one
     // cell per thread, 128 threads, 6 blocks per SM (85 registers, no spills).
     if (kNoise) shape = 4;
     const Shape sh = kShapes[shape];
     const std::int64_t units = std::max<std::int64_t>(1, a.n / sh.cells);
     const std::int64_t want = (units + sh.block - 1) / sh.block;
-    const std::int64_t cap = static_cast<std::int64_t>(sms) * sh.min_blocks * 4;
-    const int grid = static_cast<int>(std::max<std::int64_t>(1, std::min(want, cap)));
+    // One thread per unit, however many waves: a finished block is replaced at
+    // once, while a grid of resident blocks looping over the cells ends with
+    // its SMs half empty (the scheduler favours the oldest warps).  Twenty
+    // fused steps of 10^7 cells: 195 us per step against 211.
+    const unsigned grid = static_cast<unsigned>(want);
     if constexpr (kNoise) {
         astro_step_kernel<kUniform, kInput, kNoise, 1, 128, 6><<<grid, 128, 0, st>>>(a, s);
     } else {
@@ -232,7 +245,6 @@ cudaError_t launch_astro(int shape, int sms, StepArgs a, AstroArrays s, cudaStre
 // kernel (the event test is exact, so both see the same events).
 __global__ void __launch_bounds__(128, 8) astro_step_kernel_f32(StepArgs a, AstroKf kf, float* Ca,
                                                                 float* IP3, float* h) {
-    const std::int64_t step = *a.step_base + a.step_offset;
     const float ca_tot = static_cast<float>(a.u.Ca_tot), ip3_0 = static_cast<float>(a.u.IP3_0),
                 tau = static_cast<float>(a.u.tau), delta = static_cast<float>(a.u.delta),
                 weight = static_cast<float>(a.weight);
@@ -258,12 +270,14 @@ __global__ void __launch_bounds__(128, 8) astro_step_kernel_f32(StepArgs a, Astr
                 hv[j] = in ? h[i0 + j] : 0.0f;
             }
         }
+        for (int t = 0; t < a.n_steps; ++t) {
+            const std::uint64_t draw = 1000ULL + static_cast<std::uint64_t>(a.step0 + t);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float in =
-                (mix64(a.seed, static_cast<std::uint64_t>(i0 + j), 1000ULL +
-                       static_cast<std::uint64_t>(step)) >> 11) < a.p_threshold ? weight : 0.0f;
-            astro_rk4_f32(kf, ca_tot, ip3_0, tau, delta, in, 0.0f, c[j], i3[j], hv[j]);
+            for (int j = 0; j < 4; ++j) {
+                const float in = (mix64(a.seed, static_cast<std::uint64_t>(i0 + j), draw) >> 11) <
+                                         a.p_threshold ? weight : 0.0f;
+                astro_rk4_f32(kf, ca_tot, ip3_0, tau, delta, in, 0.0f, c[j], i3[j], hv[j]);
+            }
         }
         if (full) {
             reinterpret_cast<float4*>(Ca)[q] = make_float4(c[0], c[1], c[2], c[3]);
@@ -295,22 +309,27 @@ __global__ void widen_kernel(std::int64_t n, const float* __restrict__ src,
 
 // The drop-in update's kernel for its parameter form, input and noise.
 template <bool kUniform>
-cudaError_t launch_update_p(bool pending, bool noisy, int shape, int sms, const StepArgs& a,
+cudaError_t launch_update_p(bool pending, bool noisy, int shape, const StepArgs& a,
                             const AstroArrays& s, cudaStream_t st) {
     if (noisy)
-        return pending ? launch_astro<kUniform, kInputArray, true>(shape, sms, a, s, st)
-                       : launch_astro<kUniform, kInputNone, true>(shape, sms, a, s, st);
-    return pending ? launch_astro<kUniform, kInputArray, false>(shape, sms, a, s, st)
-                   : launch_astro<kUniform, kInputNone, false>(shape, sms, a, s, st);
+        return pending ? launch_astro<kUniform, kInputArray, true>(shape, a, s, st)
+                       : launch_astro<kUniform, kInputNone, true>(shape, a, s, st);
+    return pending ? launch_astro<kUniform, kInputArray, false>(shape, a, s, st)
+                   : launch_astro<kUniform, kInputNone, false>(shape, a, s, st);
 }
 
-cudaError_t launch_update(bool uniform, bool pending, bool noisy, int shape, int sms,
+cudaError_t launch_update(bool uniform, bool pending, bool noisy, int shape,
                           const StepArgs& a, const AstroArrays& s, cudaStream_t st) {
-    return uniform ? launch_update_p<true>(pending, noisy, shape, sms, a, s, st)
-                   : launch_update_p<false>(pending, noisy, shape, sms, a, s, st);
+    return uniform ? launch_update_p<true>(pending, noisy, shape, a, s, st)
+                   : launch_update_p<false>(pending, noisy, shape, a, s, st);
 }
 
-__global__ void advance_counter_kernel(std::int64_t* base, std::int64_t by) { *base += by; }
+// Steps of the Bernoulli workload per launch: all of a call's, up to 2^33
+// cell-steps (about 0.2 s), which bounds a launch's length.
+int steps_per_launch(std::int64_t n, std::int64_t left) {
+    return static_cast<int>(std::min<std::int64_t>(
+        left, std::max<std::int64_t>(1, std::min<std::int64_t>((1ll << 33) / n, 1 << 30))));
+}
 
 // ceil(p * 2^53): k * 2^-53 < p exactly when the integer k is below it
 // (p * 2^53 is exact, and an integer is below a real number exactly when it
@@ -359,14 +378,18 @@ struct AstroEngine {
     int sms = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    DevBuf Ca, IP3, h, input, Ca_tot, IP3_0, tau, inv_tau, delta, step_base;
+    DevBuf Ca, IP3, h, input, Ca_tot, IP3_0, tau, inv_tau, delta;
     // Precision study: the state rounded to float, valid while no FP64 call
     // has advanced the FP64 state since (f32_valid).
     DevBuf Ca32, IP332, h32;
     bool f32_valid = false;
     double last_ms = 0.0;
     std::int64_t last_kernels = 0;
-    int shape = 0;  // launch shape (see kShapes), set by asg_astro_autotune
+    // Launch shape (see kShapes) until asg_astro_autotune or _set_shape: one
+    // cell per thread, 64 threads, 85 registers.  Fastest or within 1 % of it at
+    // every size from 4,099 to 10^7 cells (the two-cell shapes take 2.8x at
+    // 4,099, one chain behind the other).
+    int shape = 5;
     // Per-cell parameters given at create.  When every cell has the same four
     // values (bit for bit) they are kept as scalars and no array is read.
     bool has_params = false;
@@ -381,16 +404,9 @@ struct AstroEngine {
     // the first update after the last timing read, ev1 by every update.
     bool upd_armed = false;
     std::int64_t upd_calls = 0;
-    // Captured chunk of Bernoulli steps, rebuilt when its arguments change.
-    cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0;
-    int graph_shape = -1;
-    StepArgs graph_args{};
-    bool graph_uniform = true;
 
     ~AstroEngine() {
         join_copies();
-        if (graph) cudaGraphExecDestroy(graph);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         for (int c = 0; c < kMaxPieces; ++c) {
@@ -401,12 +417,6 @@ struct AstroEngine {
         if (h2d) cudaStreamDestroy(h2d);
         if (d2h) cudaStreamDestroy(d2h);
         if (stream) cudaStreamDestroy(stream);
-    }
-
-    int grid_for(std::int64_t pairs, int block) const {
-        const std::int64_t want = (pairs + block - 1) / block;
-        const std::int64_t cap = static_cast<std::int64_t>(sms) * 16;
-        return static_cast<int>(std::max<std::int64_t>(1, std::min(want, cap)));
     }
 
     AstroArrays arrays() {
@@ -534,7 +544,6 @@ int asg_astro_create(uint32_t n, const double* Ca, const double* IP3, const doub
         upload(e->inv_tau, inv.data(), false);
     }
     upload(e->delta, delta_IP3, false);
-    if (st == ASG_OK) st = e->step_base.alloc(sizeof(std::int64_t));
     if (st == ASG_OK) {
         cudaError_t ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
         if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->h2d, cudaStreamNonBlocking);
@@ -647,7 +656,6 @@ int asg_astro_update(asg_astro* s, const double* consts, double h_step, int32_t 
     a.shared_noise = shared_noise;
     a.noise_seed = noise_seed;
     a.noise_index = noise_index;
-    a.step_base = e->step_base.as<std::int64_t>();
     if (!e->upd_armed) {
         ASG_CUDA(cudaEventRecord(e->ev0, e->stream));
         e->upd_armed = true;
@@ -665,7 +673,7 @@ int asg_astro_update(asg_astro* s, const double* consts, double h_step, int32_t 
         a.n = e->n;
         a.i0 = 0;
         ASG_CUDA(asg::launch_update(e->params_uniform, false, a.independent != 0, e->shape,
-                                    e->sms, a, e->arrays(), e->stream));
+                                    a, e->arrays(), e->stream));
         for (int c = 0; c < e->pieces(); ++c)
             ASG_CUDA(cudaEventRecord(e->ev_k[c], e->stream));
         e->upd_calls += 1;
@@ -677,7 +685,7 @@ int asg_astro_update(asg_astro* s, const double* consts, double h_step, int32_t 
             a.n = e->piece_end(c) - b;
             a.i0 = b;
             ASG_CUDA(asg::launch_update(e->params_uniform, true, a.independent != 0, e->shape,
-                                        e->sms, a, e->arrays_at(b), e->stream));
+                                        a, e->arrays_at(b), e->stream));
             ASG_CUDA(cudaEventRecord(e->ev_k[c], e->stream));
         }
         e->upd_calls += e->pieces();
@@ -731,58 +739,17 @@ int asg_astro_run_bernoulli(asg_astro* s, const double* consts, double h_step, i
     a.p = p;
     a.p_threshold = asg::bernoulli_threshold(p);
     a.weight = weight;
-    a.step_base = e->step_base.as<std::int64_t>();
 
-    // Steps run as captured chunks of up to 64 launches: kernel j of a chunk
-    // reads step = *step_base + j, and a one-thread node advances the base.
-    const int chunk = static_cast<int>(std::min<std::int64_t>(64, count));
-    cudaError_t launch_err = cudaSuccess;
-    auto launch_step = [&](int j) {
-        asg::StepArgs aj = a;
-        aj.step_offset = j;
-        const cudaError_t le =
-            uniform ? asg::launch_astro<true, asg::kInputBernoulli, false>(e->shape, e->sms, aj,
-                                                                            e->arrays(), e->stream)
-                    : asg::launch_astro<false, asg::kInputBernoulli, false>(e->shape, e->sms, aj,
-                                                                             e->arrays(), e->stream);
-        if (le != cudaSuccess) launch_err = le;
-    };
-    const bool same = e->graph != nullptr && e->graph_steps == chunk &&
-                      e->graph_uniform == (uniform != 0) && e->graph_shape == e->shape &&
-                      std::memcmp(&e->graph_args, &a, sizeof a) == 0;
-    if (!same) {
-        if (e->graph) cudaGraphExecDestroy(e->graph);
-        e->graph = nullptr;
-        cudaGraph_t g = nullptr;
-        ASG_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < chunk; ++j) launch_step(j);
-        ASG_CUDA(launch_err);
-        asg::advance_counter_kernel<<<1, 1, 0, e->stream>>>(e->step_base.as<std::int64_t>(), chunk);
-        ASG_CUDA(cudaStreamEndCapture(e->stream, &g));
-        const cudaError_t ce = cudaGraphInstantiate(&e->graph, g, 0);
-        cudaGraphDestroy(g);
-        ASG_CUDA(ce);
-        e->graph_steps = chunk;
-        e->graph_args = a;
-        e->graph_uniform = uniform != 0;
-        e->graph_shape = e->shape;
-    }
-    std::int64_t base = first;
-    ASG_CUDA(cudaMemcpyAsync(e->step_base.get(), &base, sizeof base, cudaMemcpyHostToDevice, e->stream));
-    ASG_CUDA(cudaStreamSynchronize(e->stream));
     ASG_CUDA(cudaEventRecord(e->ev0, e->stream));
-    std::int64_t done = 0;
     std::int64_t kernels = 0;
-    while (count - done >= chunk) {
-        ASG_CUDA(cudaGraphLaunch(e->graph, e->stream));
-        done += chunk;
-        kernels += chunk + 1;
-    }
-    if (done < count) {
-        // Remainder: plain launches with the base already advanced.
-        for (int j = 0; done + j < count; ++j) launch_step(j);
-        ASG_CUDA(launch_err);
-        kernels += count - done;
+    for (std::int64_t done = 0; done < count; ++kernels) {
+        a.step0 = first + done;
+        a.n_steps = asg::steps_per_launch(e->n, count - done);
+        ASG_CUDA((uniform ? asg::launch_astro<true, asg::kInputBernoulli, false>(
+                                e->shape, a, e->arrays(), e->stream)
+                          : asg::launch_astro<false, asg::kInputBernoulli, false>(
+                                e->shape, a, e->arrays(), e->stream)));
+        done += a.n_steps;
     }
     ASG_CUDA(cudaEventRecord(e->ev1, e->stream));
     ASG_CUDA(cudaEventSynchronize(e->ev1));
@@ -851,29 +818,19 @@ int asg_astro_run_bernoulli_f32(asg_astro* s, const double* consts, double h_ste
     a.p = p;
     a.p_threshold = asg::bernoulli_threshold(p);
     a.weight = weight;
-    a.step_base = e->step_base.as<std::int64_t>();
     const asg::AstroKf kf = asg::astro_k_f32(a.k);
     const std::int64_t quads = (e->n + 3) / 4;
     const int grid = static_cast<int>(std::max<std::int64_t>(
         1, std::min<std::int64_t>((quads + 127) / 128, static_cast<std::int64_t>(e->sms) * 8 * 4)));
-    std::int64_t base = first;
-    ASG_CUDA(cudaMemcpyAsync(e->step_base.get(), &base, sizeof base, cudaMemcpyHostToDevice,
-                             e->stream));
-    // Plain launches of 64-step groups, the step read from the device
-    // counter; the counter advances by a one-thread kernel after each group.
     ASG_CUDA(cudaEventRecord(e->ev0, e->stream));
-    std::int64_t done = 0, kernels = 0;
-    while (done < count) {
-        const int chunk = static_cast<int>(std::min<std::int64_t>(64, count - done));
-        for (int j = 0; j < chunk; ++j) {
-            a.step_offset = j;
-            asg::astro_step_kernel_f32<<<grid, 128, 0, e->stream>>>(
-                a, kf, e->Ca32.as<float>(), e->IP332.as<float>(), e->h32.as<float>());
-        }
-        asg::advance_counter_kernel<<<1, 1, 0, e->stream>>>(e->step_base.as<std::int64_t>(), chunk);
+    std::int64_t kernels = 0;
+    for (std::int64_t done = 0; done < count; ++kernels) {
+        a.step0 = first + done;
+        a.n_steps = asg::steps_per_launch(e->n, count - done);
+        asg::astro_step_kernel_f32<<<grid, 128, 0, e->stream>>>(
+            a, kf, e->Ca32.as<float>(), e->IP332.as<float>(), e->h32.as<float>());
         ASG_CUDA(cudaGetLastError());
-        done += chunk;
-        kernels += chunk + 1;
+        done += a.n_steps;
     }
     ASG_CUDA(cudaEventRecord(e->ev1, e->stream));
     // The FP64 state holds the widened result, for pulls and FP64 calls.
@@ -934,15 +891,15 @@ extern "C" int asg_astro_autotune(asg_astro* s, const double* consts, double h_s
     a.p = 0.01;
     a.p_threshold = asg::bernoulli_threshold(a.p);
     a.weight = 0.2;
-    a.step_base = e->step_base.as<std::int64_t>();
     int best = e->shape;
     float best_ms = 1e30f;
     for (int shape = 0; shape < asg::kNumShapes; ++shape) {
         for (int rep = 0; rep < 2; ++rep) {  // first pass warms up
             ASG_CUDA(cudaEventRecord(e->ev0, e->stream));
-            for (int j = 0; j < steps; ++j) {
-                a.step_offset = j;
-                ASG_CUDA((asg::launch_astro<true, asg::kInputBernoulli, false>(shape, e->sms, a,
+            for (int done = 0; done < steps; done += a.n_steps) {
+                a.step0 = done;
+                a.n_steps = asg::steps_per_launch(e->n, steps - done);
+                ASG_CUDA((asg::launch_astro<true, asg::kInputBernoulli, false>(shape, a,
                                                                                 arr, e->stream)));
             }
             ASG_CUDA(cudaEventRecord(e->ev1, e->stream));
@@ -1095,9 +1052,8 @@ extern "C" int asg_astro_update_noalloc(uint32_t n, double* Ca, double* IP3, dou
                          "asg_astro_update_noalloc: a CUDA error from earlier work is pending "
                          "on this thread (%s: %s); nothing was launched",
                          cudaGetErrorName(pending), cudaGetErrorString(pending));
-    int dev = 0, sms = 148;
+    int dev = 0;
     ASG_CUDA(cudaGetDevice(&dev));
-    ASG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     double* inv_tau = nullptr;
     ASG_TRY(asg::noalloc_scratch(dev, &inv_tau));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1118,7 +1074,7 @@ extern "C" int asg_astro_update_noalloc(uint32_t n, double* Ca, double* IP3, dou
     // Shape 1: one cell per thread with 8-byte accesses, so caller arrays need
     // no more than double alignment.
     ASG_CUDA(a.independent
-                 ? (asg::launch_astro<false, asg::kInputArrayZero, true>(1, sms, a, arr, st))
-                 : (asg::launch_astro<false, asg::kInputArrayZero, false>(1, sms, a, arr, st)));
+                 ? (asg::launch_astro<false, asg::kInputArrayZero, true>(1, a, arr, st))
+                 : (asg::launch_astro<false, asg::kInputArrayZero, false>(1, a, arr, st)));
     return ASG_OK;
 }
