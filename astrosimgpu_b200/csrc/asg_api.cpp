@@ -120,6 +120,7 @@ int autotune_engine(Engine& e, int32_t steps, asg_engine_opts* chosen) {
     for (std::size_t i = 0; i < e.insts.size(); ++i) {
         Instance& I = *e.insts[i];
         Snap& s = snaps[i];
+        ASG_TRY(e.sync_arena(I));
         ASG_TRY(s.copy.alloc(I.arena_bytes, false));
         ASG_CUDA(cudaMemcpyAsync(s.copy.get(), I.arena.get(), I.arena_bytes,
                                  cudaMemcpyDeviceToDevice, e.stream));
@@ -156,6 +157,7 @@ int autotune_engine(Engine& e, int32_t steps, asg_engine_opts* chosen) {
             I.n_spikes = s.ns;
         }
         ASG_CUDA(cudaStreamSynchronize(e.stream));
+        for (auto& p : e.insts) ASG_TRY(e.arena_restored(*p));
         return ASG_OK;
     };
     const int block0 = e.cfg.block, chunk0 = e.cfg.chunk_steps, mode0 = e.cfg.use_graphs;
@@ -309,7 +311,7 @@ int asg_checkpoint(asg_network* net, void* host_buf, uint64_t bytes) {
     asg::Instance* I = h->eng->find(h->id);
     if (bytes < I->arena_bytes + sizeof(int64_t))
         return asg::fail(ASG_ERR_OVERFLOW, "checkpoint needs %zu bytes", I->arena_bytes + 8);
-    ASG_CUDA(cudaStreamSynchronize(h->eng->stream));
+    ASG_TRY(h->eng->sync_arena(*I));
     std::memcpy(host_buf, &I->step, sizeof(int64_t));
     ASG_CUDA(cudaMemcpy(static_cast<char*>(host_buf) + 8, I->arena.get(), I->arena_bytes,
                         cudaMemcpyDeviceToHost));
@@ -331,7 +333,7 @@ int asg_restore(asg_network* net, const void* host_buf, uint64_t bytes) {
     I->spikes.clear();
     I->dev.noise_from = I->step;  // noise terms drawn afresh at the first step
     h->eng->mark_side_prime();
-    return ASG_OK;
+    return h->eng->arena_restored(*I);
 }
 
 int asg_destroy(asg_network* net) {

@@ -681,6 +681,32 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
         const int want = static_cast<int>((sic_mx + kSicEdgesPerPart - 1) / kSicEdgesPerPart);
         D.sic_parts = std::max(1, std::min({want, kMaxSicParts, D.d_a2n - 1}));
     }
+    D.fac_slots = D.slots;
+    D.fany_slots = D.slots + 1;
+    D.fany_ahead = 1;
+    // Steps per launch: the spikes of a launch are pushed by the next one and
+    // must land before a third reads them; the SIC factors a launch reads
+    // must be older than it (one step more where the current is formed a step
+    // ahead).  Side batches cover kSicBatchSteps steps from a multiple of it,
+    // so launches must not straddle one, and a batch must not read factor
+    // rows that the launch beside it writes.
+    I.span_max = 1;
+    if (D.deferred_push) {
+        int L = std::min({kMaxSpan, D.d_e / 2, D.d_i / 2});
+        if (D.sic_side) {
+            L = std::min(L, D.slots >= 2 * kSicBatchSteps ? kSicBatchSteps : kSicBatchSteps / 2);
+        } else if (NA > 0) {
+            L = D.sic_parts > 1 ? 1 : std::min(L, D.d_a2n - (D.fused_sic ? 0 : 1));
+        }
+        for (const asg_csr* c : {&d.exc_primary, &d.inh_primary, &d.neuron_astro}) {
+            const std::uint32_t* rs = rs_of(*c);  // a spike record holds a row length in 28 bits
+            if (first_bad(c->n_sources, [&](std::uint32_t i) {
+                    return rs[i + 1] - rs[i] >= (1u << 28);
+                }) < c->n_sources)
+                L = 1;
+        }
+        I.span_max = std::max(1, L);
+    }
     SicHost sic = make_sic(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N,
                            static_cast<std::uint32_t>(D.sic_parts), D.sic_npad);
 
@@ -785,7 +811,6 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
     {
         char* base = I.arena.as<char>();
         std::size_t off = 0;
-        std::vector<char> zeros;
         for (const Seg& s : segs) {
             *static_cast<void**>(s.dst) = base + off;
             if (s.bytes > 0) {
@@ -799,7 +824,36 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
             }
             off += align256(std::max<std::size_t>(s.bytes, 1));
         }
+        I.fac_off = static_cast<std::size_t>(reinterpret_cast<char*>(D.fac) - base);
+        I.fany_off = static_cast<std::size_t>(reinterpret_cast<char*>(D.fac_any) - base);
         ASG_CUDA(cudaStreamSynchronize(upload));  // host sources go out of scope
+    }
+
+    // The span buffer comes out of what the budget leaves free; without it
+    // the instance runs one step per launch.
+    if (I.span_max > 1) {
+        const std::size_t cap = static_cast<std::size_t>(N) * I.span_max;
+        const std::size_t rec = align256(2 * cap * 16);
+        const std::size_t fac = D.sic_side ? 0 : align256(static_cast<std::size_t>(D.d_a2n + kMaxSpan) * a8);
+        const std::size_t any = align256((static_cast<std::size_t>(D.d_a2n) + 2 * kMaxSpan) * 4);
+        const std::size_t bytes = 2 * rec + fac + any;
+        const std::uint64_t used = resident_bytes + total;
+        const std::uint64_t left = cfg.mem_budget > used ? cfg.mem_budget - used : 0;
+        std::size_t fr = 0, tot = 0;
+        ASG_CUDA(cudaMemGetInfo(&fr, &tot));
+        if (fr >= bytes && fr - bytes >= left && I.span.alloc(bytes, false) == ASG_OK) {
+            char* p = I.span.as<char>();
+            ASG_CUDA(cudaMemsetAsync(p + 2 * rec, 0, fac + any, upload));
+            ASG_CUDA(cudaStreamSynchronize(upload));
+            D.span_meta = reinterpret_cast<std::uint32_t*>(p);
+            D.span_val = reinterpret_cast<double*>(p + rec);
+            D.span_cap = cap;
+            I.span_fac = reinterpret_cast<double*>(p + 2 * rec);
+            I.span_fany = reinterpret_cast<std::uint32_t*>(p + 2 * rec + fac);
+        } else {
+            clear_error();
+            I.span_max = 1;
+        }
     }
 
     // Recording and spike-log buffers (mapped host memory, two parities).
@@ -886,6 +940,31 @@ int Engine::rebuild() {
     ASG_CUDA(cudaStreamSynchronize(stream));
     drop_graphs();
     const int B = cfg.block;
+    // Steps per launch: the least any instance allows; the persistent kernel
+    // and plain launches take single steps.
+    span = cfg.use_graphs == 2 || cfg.use_graphs == -1 || B != 128 || insts.empty() ? 1 : kMaxSpan;
+    bool any_side = false;
+    for (auto& p : insts) {
+        span = std::min(span, p->span_max);
+        any_side = any_side || p->dev.sic_side;
+    }
+    if (any_side)  // a divisor of the side batch
+        while (kSicBatchSteps % span != 0) --span;
+    for (auto& p : insts) {
+        InstDev& D = p->dev;
+        D.sic_inline = span > 1 && !D.fused_sic && !D.sic_side;
+        if (!D.sic_side && p->fac_in_span != (span > 1)) {
+            ASG_TRY(copy_factors(*p, span > 1));
+            p->fac_in_span = span > 1;
+        }
+        double* arena_fac = reinterpret_cast<double*>(p->arena.as<char>() + p->fac_off);
+        std::uint32_t* arena_fany = reinterpret_cast<std::uint32_t*>(p->arena.as<char>() + p->fany_off);
+        D.fac = p->fac_in_span ? p->span_fac : arena_fac;
+        D.fac_any = p->fac_in_span ? p->span_fany : arena_fany;
+        D.fac_slots = p->fac_in_span ? D.d_a2n + kMaxSpan : D.slots;
+        D.fany_slots = p->fac_in_span ? D.d_a2n + 2 * kMaxSpan : D.slots + 1;
+        D.fany_ahead = p->fac_in_span ? kMaxSpan : 1;
+    }
     work.clear();
     order.clear();
     // Push and SIC blocks first (longest dependent chains), then neurons, then
@@ -899,7 +978,8 @@ int Engine::rebuild() {
                                     : role == 1 ? kRoleSic
                                     : role == 2 ? kRoleNeuron
                                                 : kRoleAstro;
-            if (r == kRoleSic && (D.fused_sic || (D.sic_side && cfg.use_graphs != 2))) continue;
+            if (r == kRoleSic && (D.fused_sic || D.sic_inline || (D.sic_side && cfg.use_graphs != 2)))
+                continue;
             if (r == kRolePush) {
                 if (!D.deferred_push) continue;
                 for (int pb = 0; pb < D.push_blocks; ++pb)
@@ -943,14 +1023,14 @@ int Engine::rebuild() {
         if (cap > cap_insts) {
             const std::size_t c2 = std::max(cap, cap_insts * 2);
             ASG_TRY(d_insts.alloc(c2 * sizeof(InstDev)));
-            ASG_TRY(d_stats.alloc(c2 * 8 * sizeof(unsigned long long)));
+            ASG_TRY(d_stats.alloc(c2 * kStatWords * sizeof(unsigned long long)));
             for (int p = 0; p < 2; ++p) {
                 if (h_insts[p]) cudaFreeHost(h_insts[p]);
                 if (h_stats[p]) cudaFreeHost(h_stats[p]);
                 h_insts[p] = nullptr;
                 h_stats[p] = nullptr;
                 ASG_CUDA(cudaHostAlloc(&h_insts[p], c2 * sizeof(InstDev), cudaHostAllocDefault));
-                ASG_CUDA(cudaHostAlloc(&h_stats[p], c2 * 8 * sizeof(unsigned long long),
+                ASG_CUDA(cudaHostAlloc(&h_stats[p], c2 * kStatWords * sizeof(unsigned long long),
                                        cudaHostAllocDefault));
             }
             cap_insts = c2;
@@ -966,24 +1046,26 @@ int Engine::rebuild() {
     if (!side_work.empty())
         ASG_CUDA(cudaMemcpyAsync(d_side_work.get(), side_work.data(),
                                  side_work.size() * sizeof(Work), cudaMemcpyHostToDevice, stream));
-    ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, cap_insts * 8 * sizeof(unsigned long long), stream));
+    ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, cap_insts * kStatWords * sizeof(unsigned long long),
+                             stream));
     ASG_CUDA(cudaStreamSynchronize(stream));
-    // Step kernel form: a step of more than two waves of the latency form
-    // (4 blocks of 128 threads per SM) is throughput-bound, and the
-    // high-occupancy form (6 blocks per SM, some spilled registers) runs it
-    // faster; a smaller step is bound by its dependent round trips, which
-    // the latency form keeps fewest.
-    wide = cfg.block == 128 &&
-           (cfg.occupancy == 2 ||
-            (cfg.occupancy == 0 && work.size() > static_cast<std::size_t>(2 * 4 * sms)));
-    // The high-occupancy form runs as one wave of resident blocks, each
-    // taking several work items (no per-item block launch or descriptor
-    // staging after its first).
+    // Step kernel form: a large step is throughput-bound and the wide form runs
+    // it faster; a smaller one is bound by its dependent round trips, which the
+    // latency form keeps fewest.  Launches of one step: the line lies at two
+    // waves of the latency form (4 blocks of 128 threads per SM).  Launches of
+    // several: a little above one wave of it (3 per SM); per step, latency and
+    // wide form: 25,000 neurons (490 items) 3.17 and 3.59 us, 30,000 (588) 4.22
+    // and 3.60, 60,000 7.47 and 6.01.
+    const std::size_t line = span > 1 ? static_cast<std::size_t>(7 * sms / 2)
+                                      : static_cast<std::size_t>(8 * sms);
+    wide = cfg.block == 128 && (cfg.occupancy == 2 || (cfg.occupancy == 0 && work.size() > line));
+    // The large forms run as one wave of resident blocks, each taking several
+    // work items (no per-item block launch or descriptor staging after its
+    // first).
     wide_grid = 0;
-    if (wide && cfg.item_loop) {
-        const int nb = step_wide_blocks_per_sm();
-        if (nb > 0) wide_grid = nb * sms;
-    }
+    if (wide && cfg.item_loop)
+        wide_grid = sms * step_blocks_per_sm(span > 1 ? StepForm::kSpanWide : StepForm::kWide,
+                                             cfg.astro_fp32);
     persistent_grid = 0;
     if (cfg.use_graphs == 2 && !work.empty()) {
         const int cap = persistent_blocks(B);
@@ -1038,49 +1120,125 @@ int Engine::capture_graph(int steps) {
     return ASG_OK;
 }
 
+// The launches of a chunk of `steps` steps.  Several steps per launch: the
+// last launch takes one step and leaves its spikes in the arena's list; the
+// one before it clears that list, so there must be a first launch, which
+// pushes from it, before that.
+std::vector<Span> Engine::plan(int steps) const {
+    std::vector<Span> v;
+    if (span == 1 || steps < span + 2) {
+        for (int k = 0; k < steps; ++k) v.push_back(Span{k, 1, k - 1, 0, 3, 3, -1, 0});
+        return v;
+    }
+    for (int k = 0; k < steps - 1; k += span)
+        v.push_back(Span{k, std::min(span, steps - 1 - k), 0, 0, 0, 0, -1, 0});
+    v.push_back(Span{steps - 1, 1, 0, 0, 0, 0, -1, 0});
+    const int m = static_cast<int>(v.size());
+    for (int i = 0; i < m; ++i) {
+        v[i].i = i;
+        v[i].kprev = i == 0 ? -1 : v[i - 1].k;
+        v[i].src = i == 0 ? 3 : (i - 1) % 3;
+        v[i].dst = i == m - 1 ? 3 : i % 3;
+        v[i].clear = i < m - 2 ? (i + 1) % 3 : -1;
+        v[i].clear_arena = i == m - 2;
+    }
+    return v;
+}
+
 // The launches of `steps` steps on the engine stream, with the side-stream
 // SIC batches: before step k (k a multiple of kSicBatchSteps) the side stream
 // waits for the steps before k and runs the batch for the arrival steps
-// step0+k+lead..; the step k+lead (the first reader, lead the smallest over
-// the instances) waits for that batch.  The side stream joins the engine
-// stream at the end, so nothing of a chunk outlives it.  The first step of a
-// chunk follows the descriptor copy: no early (programmatic) launch for it.
+// step0+k+lead..; the launch of step k+lead (the first reader, lead the
+// smallest over the instances) waits for that batch.  The side stream joins
+// the engine stream at the end, so nothing of a chunk outlives it.  The first
+// launch of a chunk follows the descriptor copy: no early (programmatic)
+// launch for it.
 cudaError_t Engine::issue_steps(int steps) {
     NvtxRange nvtx("step chain: arrival application, background input, update astrocytes, "
                    "update neurons, spike delivery, SIC gather+deliver");
     const bool side_on = !side_work.empty();
     const int G = kSicBatchSteps;
+    const StepForm form = span > 1 ? (wide ? StepForm::kSpanWide : StepForm::kSpan)
+                                   : (wide ? StepForm::kWide : StepForm::kLatency);
     cudaError_t e = cudaSuccess;
     if (side_on) {
         e = cudaEventRecord(ev_side_fork, stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(side, ev_side_fork, 0);
     }
-    for (int k = 0; k < steps && e == cudaSuccess; ++k) {
-        if (side_on && k % G == 0) {
-            cudaEvent_t before = ev_side_pre[(k / G) % kSideEvents];
-            cudaEvent_t done = ev_side_done[(k / G) % kSideEvents];
+    for (const Span& sp : plan(steps)) {
+        if (e != cudaSuccess) break;
+        if (side_on && sp.k % G == 0) {
+            cudaEvent_t before = ev_side_pre[(sp.k / G) % kSideEvents];
+            cudaEvent_t done = ev_side_done[(sp.k / G) % kSideEvents];
             e = cudaEventRecord(before, stream);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(side, before, 0);
             if (e == cudaSuccess)
                 e = launch_sic_batch(d_insts.as<InstDev>(), d_side_work.as<Work>(),
-                                     static_cast<int>(side_work.size()), cfg.block, k, side);
+                                     static_cast<int>(side_work.size()), cfg.block, sp.k, side);
             if (e == cudaSuccess) e = cudaEventRecord(done, side);
         }
-        // (A step that waits for a batch still launches early: it reads the
+        // (A launch that waits for a batch still launches early: it reads the
         // SIC values after griddepcontrol.wait, and the batch is a completed
         // prerequisite by then whichever way the wait is honoured.)
-        if (side_on && k >= side_lead && (k - side_lead) % G == 0 && e == cudaSuccess)
-            e = cudaStreamWaitEvent(stream, ev_side_done[((k - side_lead) / G) % kSideEvents], 0);
+        for (int k = sp.k; side_on && k < sp.k + sp.cnt && e == cudaSuccess; ++k)
+            if (k >= side_lead && (k - side_lead) % G == 0)
+                e = cudaStreamWaitEvent(stream, ev_side_done[((k - side_lead) / G) % kSideEvents], 0);
         if (e == cudaSuccess)
             e = launch_step(d_insts.as<InstDev>(), d_work.as<Work>(), static_cast<int>(work.size()),
-                            cfg.block, k, cfg.pdl && k > 0, wide, wide_grid, cfg.astro_fp32,
-                            stream);
+                            cfg.block, sp, cfg.pdl && sp.k > 0, form, wide ? wide_grid : 0,
+                            cfg.astro_fp32, stream);
     }
     if (side_on && e == cudaSuccess) {
         e = cudaEventRecord(ev_side_join, side);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ev_side_join, 0);
     }
     return e;
+}
+
+// Copies the SIC factors of the emission steps a later step can still read
+// (and their flags) between the arena's rows and the span buffer's.
+int Engine::copy_factors(Instance& I, bool to_span) {
+    const InstDev& D = I.dev;
+    if (I.step == 0 || D.NA == 0) return ASG_OK;  // nothing emitted, all zero
+    const std::size_t row = static_cast<std::size_t>(D.NA) * 8;
+    char* arena = I.arena.as<char>() + I.fac_off;
+    char* sp = reinterpret_cast<char*>(I.span_fac);
+    const int S = D.slots, F = D.d_a2n + kMaxSpan, AS = D.slots + 1, AF = D.d_a2n + 2 * kMaxSpan;
+    std::vector<std::uint32_t> a(AS, 0u), f(AF, 0u);
+    std::uint32_t* arena_any = reinterpret_cast<std::uint32_t*>(I.arena.as<char>() + I.fany_off);
+    if (to_span)
+        ASG_CUDA(cudaMemcpy(a.data(), arena_any, AS * 4, cudaMemcpyDeviceToHost));
+    else
+        ASG_CUDA(cudaMemcpy(f.data(), I.span_fany, AF * 4, cudaMemcpyDeviceToHost));
+    for (std::int64_t e = std::max<std::int64_t>(0, I.step - D.d_a2n); e < I.step; ++e) {
+        char* x = arena + static_cast<std::size_t>(e % S) * row;
+        char* y = sp + static_cast<std::size_t>(e % F) * row;
+        ASG_CUDA(cudaMemcpyAsync(to_span ? y : x, to_span ? x : y, row, cudaMemcpyDeviceToDevice,
+                                 stream));
+        if (to_span)
+            f[e % AF] = a[e % AS];
+        else
+            a[e % AS] = f[e % AF];
+    }
+    if (to_span)
+        ASG_CUDA(cudaMemcpy(I.span_fany, f.data(), AF * 4, cudaMemcpyHostToDevice));
+    else
+        ASG_CUDA(cudaMemcpy(arena_any, a.data(), AS * 4, cudaMemcpyHostToDevice));
+    ASG_CUDA(cudaStreamSynchronize(stream));
+    return ASG_OK;
+}
+
+int Engine::sync_arena(Instance& I) {
+    ASG_TRY(finish_pending());
+    ASG_CUDA(cudaStreamSynchronize(stream));
+    return I.fac_in_span ? copy_factors(I, false) : ASG_OK;
+}
+
+int Engine::arena_restored(Instance& I) {
+    if (!I.fac_in_span) return ASG_OK;
+    if (I.step == 0)
+        ASG_CUDA(cudaMemset(I.span_fany, 0, (I.dev.d_a2n + 2 * kMaxSpan) * 4));
+    return copy_factors(I, true);
 }
 
 // SIC values of the arrival steps step0 .. step0+lead-1 of every side
@@ -1107,9 +1265,10 @@ int Engine::launch_chunk(int parity, int steps) {
         InstDev D = I.dev;
         D.step0 = I.step;
         D.end_step = std::min<std::int64_t>(I.end, I.step + steps);
-        unsigned long long* st = d_stats.as<unsigned long long>() + s * 8;
+        unsigned long long* st = d_stats.as<unsigned long long>() + s * kStatWords;
         D.spike_log_n = st;
         D.counters = st + 1;
+        D.span_packed = st + 16;
         D.spike_log = I.log_d[parity];
         double* r = I.rec_d[parity];
         const std::size_t R = I.rec_rows;
@@ -1141,14 +1300,13 @@ int Engine::launch_chunk(int parity, int steps) {
     } else {
         ASG_CUDA(issue_steps(steps));
     }
-    const int launched = persistent_grid > 0 ? 1 : steps;
+    const int launched = persistent_grid > 0 ? 1 : static_cast<int>(plan(steps).size());
     last_kernels += launched;
     launched_kernels += launched;
-    ASG_CUDA(cudaMemcpyAsync(h_stats[parity], d_stats.get(),
-                             insts.size() * 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+    const std::size_t stat_bytes = insts.size() * kStatWords * sizeof(unsigned long long);
+    ASG_CUDA(cudaMemcpyAsync(h_stats[parity], d_stats.get(), stat_bytes, cudaMemcpyDeviceToHost,
                              stream));
-    ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, insts.size() * 8 * sizeof(unsigned long long),
-                             stream));
+    ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, stat_bytes, stream));
     ASG_CUDA(cudaEventRecord(ev_chunk[parity], stream));
     pending[parity] = true;
     launched_insts[parity] = insts.size();
@@ -1175,7 +1333,7 @@ int Engine::collect(int parity) {
     for (std::size_t s = 0; s < n_launched; ++s) {
         Instance& I = *insts[s];
         const InstDev& D = I.dev;
-        const unsigned long long* c = st + s * 8;
+        const unsigned long long* c = st + s * kStatWords;
         if (c[4] != 0)
             return fail(ASG_ERR_OVERFLOW,
                         "instance %d: %llu spikes did not fit the %u-entry chunk log; use a "

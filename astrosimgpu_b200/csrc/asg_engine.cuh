@@ -1,18 +1,22 @@
 // Device data layout of the network engine (one descriptor per instance) and
 // the fused per-timestep kernel.
 //
-// One kernel launch advances every resident instance by one step.  Its
-// blocks are typed by a work table built on the host:
+// One kernel launch advances every resident instance by one step or, where
+// the delays allow, by several (see Span).  Its blocks are typed by a work
+// table built on the host:
+//   PUSH    the out-edges of the spikes of the launch before, into the arrival
+//           rings of later steps;
 //   NEURON  arrivals (exc/inh rings, SIC), Poisson drive, noise, AdEx RK4,
-//           spike test, STP update of the spiking source and the push of its
-//           out-edges into the arrival rings of later steps;
+//           spike test, STP update of the spiking source and its append to the
+//           launch's spike list (with a one-step delay: its push);
 //   ASTRO   arrivals (neuron->astrocyte ring), Poisson drive, noise, Li-Rinzel
 //           RK4, SIC factor of the step;
-//   SIC     (only when the SIC delay is >= 2 steps) the SIC current arriving
-//           at the NEXT step, summed from the factors of its emission step.
+//   SIC     (launches of one step, when the SIC delay is >= 2 steps) the SIC
+//           current arriving at the NEXT step, summed from the factors of its
+//           emission step.
 // No role waits on another inside a launch: every cross-cell read is of data
-// written by an earlier launch (delays are >= 1 step), so one launch per step
-// is the only synchronisation, and K steps are one captured CUDA graph.
+// written by an earlier launch, so the launch boundary is the only
+// synchronisation, and the launches of K steps are one captured CUDA graph.
 //
 // Exact, reproducible arrivals without floating-point atomics
 // ----------------------------------------------------------
@@ -77,6 +81,7 @@ constexpr std::uint16_t kNoHelper = 0xFFFFu;
 constexpr int kListCap = 4;      // arrivals per (slot, target) held in the short list
 constexpr int kMaxSicParts = 8;  // most parts a target's SIC chain is cut into
 constexpr int kHeaderStride = 16;  // u64 words between spike-list headers (128 bytes)
+constexpr int kMaxSpan = 8;        // most steps one launch advances
 constexpr int kSicBatchSteps = 8;  // arrival steps per side-stream SIC batch
 constexpr int kSicRing = 32;       // SIC value slots of an instance with side batches
 
@@ -158,14 +163,25 @@ struct InstDev {
     // block must not share an L2 sector, or the reads queue behind the atomics.
     unsigned long long* spk_packed;
     std::uint32_t* spk_meta;           // [3][N][4]: n2a row start (~0: inhibitory source),
-                                       // edge offset, row0 start, row0 length
+                                       // edge offset, row0 start, row0 length | step << 28
+                                       // (the spike's step in its launch)
     double* spk_val;                   // [3][N][2]: exc or inh set value, n2a value
+    // The same for launches of several steps (see Span): three headers, two
+    // lists of span_cap records.
+    unsigned long long* span_packed;
+    std::uint32_t* span_meta;
+    double* span_val;
+    std::uint64_t span_cap;
     // SIC: sliced ELL over virtual targets v = part * sic_npad + target,
     // factors per emission slot, partial sums between parts, final values.
     // With sic_side the currents are computed off the step kernels, by
     // side-stream batches: the batch launched before step s (s a multiple of
     // kSicBatchSteps in the chunk) covers the arrival steps s+sic_lead ..
     // s+sic_lead+kSicBatchSteps-1, one whole chain per thread (P = 1).
+    // sic_inline: launches of several steps of an instance with the SIC role's
+    // schedule (the current arriving at step s+1 is formed during step s): the
+    // neuron thread forms it and leaves the last one in sic_val.
+    std::int32_t sic_inline;
     std::int32_t sic_side;
     std::int32_t sic_lead;
     std::int32_t sic_ring;          // slots of sic_val, a power of two
@@ -173,12 +189,19 @@ struct InstDev {
     std::uint32_t sic_npad;         // N rounded up to a multiple of 32
     const std::uint32_t* sic_soff;  // [P*sic_npad/32+1] entry offset of each 32-target slice
     const std::uint32_t* sic_ent;   // astro << 8 | mult
-    double* fac;                    // [slots][NA]
-    // fac_any[e % (slots + 1)] != 0: some factor of emission step e is
-    // non-zero.  Set by the astrocyte role, cleared one step ahead by the
-    // instance's first astrocyte block; a fused SIC sum of an arrival whose
-    // emission had none is the +0.0 it would add up to, without its loads.
-    std::uint32_t* fac_any;         // [slots + 1]
+    // Factors by emission step: slots rows in the arena, or, while launches
+    // advance several steps, d_a2n + kMaxSpan rows in the instance's span
+    // buffer (a launch writes the rows of its own steps while it reads those
+    // of steps up to d_a2n before them).
+    double* fac;                    // [fac_slots][NA]
+    std::int32_t fac_slots;
+    // fac_any[e % fany_slots] != 0: some factor of emission step e is
+    // non-zero.  Set by the astrocyte role, cleared fany_ahead steps ahead
+    // (the longest launch) by the instance's first astrocyte block; a fused
+    // SIC sum of an arrival whose emission had none is the +0.0 it would add
+    // up to, without its loads.
+    std::int32_t fany_slots, fany_ahead;
+    std::uint32_t* fac_any;
     double* sic_part;               // [2][P-1][sic_npad] partial sums, by step parity
     double* sic_val;                // [sic_ring][N], slot = arrival step % sic_ring
     // outputs (host-mapped memory)
@@ -191,6 +214,33 @@ struct InstDev {
     std::uint32_t rec_astro_max, rec_neuron_max, rec_rows;  // rows held in the ring below
     double *rec_Ca, *rec_IP3, *rec_V, *rec_Isic;             // [rec_rows][max]
     unsigned long long* counters;  // spike_edges, sic_edges, spikes, overflow
+};
+
+// The steps of one launch: [step0 + k, step0 + k + cnt).
+//
+// A spike travels at least min(d_e, d_i) steps and a SIC factor d_a2n, so what
+// the steps of a launch read was written by earlier launches as long as a
+// launch and the one after it (which pushes the launch's spikes) together
+// cover no more than the spike delay, and a launch no more than the SIC
+// delay.  A thread then advances its cell by all cnt steps with the state in
+// registers, and the launch boundary, the descriptor staging and the state's
+// round trip are paid once per launch instead of once per step.  With delays
+// of ten steps (five per launch), per step: 500 neurons 3.32 -> 2.05 us (a step
+// is now its RK4 chain, ~1.1 us, the rest of its loop and a fifth of a launch
+// boundary), 10,000 4.1 -> 2.5, 200,000 25.8 -> 19.2, 10^6 118 -> 82.
+//
+// Spike lists: list 3 is the arena's, by step (the launches of one step);
+// 0..2 are span headers i % 3 with the records in span list i & 1.  A chunk of
+// several-step launches i = 0 .. m-1 (m >= 3) pushes from the arena list in
+// launch 0 and ends with a launch of one step that appends to the arena list
+// again, so that between chunks the arena alone holds the instance's state.
+struct Span {
+    int k, cnt;
+    int kprev;       // first step of the launch before (its spikes are pushed now)
+    int i;           // launch index in the chunk (span chunks)
+    int src, dst;    // spike lists pushed from and appended to
+    int clear;       // span header this launch clears (-1: none; arena rotation for dst 3)
+    int clear_arena; // clears the arena headers (the launch before the chunk's last)
 };
 
 // Barrier words of the persistent chunk kernel (device memory, zeroed).
@@ -214,15 +264,18 @@ cudaError_t launch_chunk_persistent(const InstDev* insts, const Work* work, int 
 cudaError_t launch_sic_batch(const InstDev* insts, const Work* work, int n_work, int block, int k,
                              cudaStream_t stream);
 
-// One step launch; with `pdl` the launch may start while the previous kernel
-// of the stream is still running (the kernel waits for it before any access
-// to instance state).
-// `wide`: the high-occupancy form (block 128 only; same arithmetic).
-// One step launch over the work table.  max_grid > 0 caps the grid (blocks
-// then run several work items each); 0 launches one block per item.
-cudaError_t launch_step(const InstDev* insts, const Work* work, int n_work, int block, int k,
-                        bool pdl, bool wide, int max_grid, bool f32, cudaStream_t stream);
-// Resident blocks per SM of the high-occupancy step kernel form (128 threads).
-int step_wide_blocks_per_sm();
+// Forms of the step kernel: launches of one step (few round trips; high
+// occupancy) and launches of several steps (the same two).
+enum class StepForm { kLatency, kWide, kSpan, kSpanWide };
+
+// One launch of the steps of `sp` over a range of the work table; with `pdl`
+// the launch may start while the previous kernel of the stream is still
+// running (the kernel waits for it before any access to instance state).
+// max_grid > 0 caps the grid (the wide forms' blocks then run several work
+// items each); 0 launches one block per item.
+cudaError_t launch_step(const InstDev* insts, const Work* work, int n_work, int block, Span sp,
+                        bool pdl, StepForm form, int max_grid, bool f32, cudaStream_t stream);
+// Resident blocks of 128 threads per SM of a kernel form.
+int step_blocks_per_sm(StepForm form, bool f32);
 
 }  // namespace asg

@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <string>
@@ -29,6 +30,15 @@ struct Instance {
     InstDev dev{};             // host copy of the device descriptor
     DevBuf arena;              // every device array of the instance
     std::size_t arena_bytes = 0;
+    // Launches of several steps (see Span): the most steps this instance's
+    // delays allow (1: none), their spike lists and SIC factor rows, and
+    // whether the factors live there now or in the arena.
+    int span_max = 1;
+    DevBuf span;
+    double* span_fac = nullptr;
+    std::uint32_t* span_fany = nullptr;
+    bool fac_in_span = false;
+    std::size_t fac_off = 0, fany_off = 0;  // the arena's factor rows and flags
     std::int64_t step = 0;     // next step to run
     std::int64_t end = INT64_MAX;
     bool done() const { return step >= end; }
@@ -114,7 +124,7 @@ public:
     std::int64_t chunks = 0;
     double chunk_device_ms = 0.0;  // sum over collected chunks (serving)
     std::int64_t launched_kernels = 0;
-    std::uint64_t resident_bytes = 0;
+    std::atomic<std::uint64_t> resident_bytes{0};  // also read by a preparing thread
     cudaStream_t stream = nullptr;
     int sms = 148;
 
@@ -122,6 +132,11 @@ public:
     // step .. step+lead-1 (after a restore: the ring may come from another
     // launch mode).
     void mark_side_prime() { side_prime = true; }
+    // Brings the factor rows of the instance's arena up to date (its state
+    // between chunks is then all in the arena).
+    int sync_arena(Instance& I);
+    // The arena was overwritten (a restore): takes the factor rows from it.
+    int arena_restored(Instance& I);
 
     int set_block(int block);
     int set_chunk(int chunk);
@@ -129,7 +144,10 @@ public:
 
 private:
     int rebuild();          // work table + graph after the instance set changed
+    std::vector<Span> plan(int steps) const;  // the launches of a chunk
     cudaError_t issue_steps(int steps);  // step launches + side-stream SIC batches
+    int copy_factors(Instance& I, bool to_span);
+    int span = 1;  // most steps per launch
     int launch_chunk(int parity, int steps);
     int collect(int parity);
     int finish_pending();
@@ -137,7 +155,10 @@ private:
     DevBuf d_insts, d_work;
     InstDev* h_insts[2] = {nullptr, nullptr};  // pinned staging
     unsigned long long* h_stats[2] = {nullptr, nullptr};  // pinned: per inst log_n + counters
-    DevBuf d_stats;        // [n][8]: log_n, spike_edges, sic_edges, spikes, overflow
+    // [n][kStatWords]: log_n, spike_edges, sic_edges, spikes, overflow, then the
+    // span spike-list headers; cleared together at the end of each chunk
+    static constexpr std::size_t kStatWords = 16 + 3 * kHeaderStride;
+    DevBuf d_stats;
     DevBuf d_barrier;      // GridBarrier of the persistent chunk kernel
     unsigned* h_barrier_err[2] = {nullptr, nullptr};  // pinned copy of its error word
     int persistent_grid = 0;

@@ -48,13 +48,15 @@ struct StepInfo {
     std::int64_t step;
     std::uint32_t slot;        // ring slot read this step: step % slots
     std::uint32_t fslot;       // factor slot of the SIC arriving now (fused SIC)
+    std::uint32_t eslot;       // factor slot this step's astrocytes write
     // SIC role: part p works on arrival step+P-p; bit p of sic_due says
     // that arrival takes SIC, sic_slot[p] is its factor slot
     std::uint32_t sic_due;
     std::uint32_t sic_slot[kMaxSicParts];
-    std::uint32_t push_e, push_i;          // deferred push of step-1's spikes
+    // deferred push: ring slots of the first step of the launch before
+    std::uint32_t push_e, push_i;
     std::uint32_t now_e, now_i;            // in-block push of this step's spikes
-    std::uint32_t ls, ls_prev, ls_next;    // spike-list slots of step, step-1, step+1
+    std::uint32_t ls, ls_prev, ls_next;    // arena spike lists of step, step-1, step+1
     std::uint32_t rec_row;
     std::uint64_t noise_e, noise_i, noise_a;  // noise draw indices
     std::int32_t sic_now, fac_now, rec_now;
@@ -65,18 +67,24 @@ struct StepInfo {
     std::int32_t fany_now, fany_next, fany_read;
 };
 
-// Computed by warp 0 of the block: each lane forms one quotient and
-// remainder (of a step offset by a period), so the whole set costs the
-// latency of one 64-bit division instead of some twenty in a row.
-__device__ void make_step_info(const InstDev& I, std::int64_t step, StepInfo& S) {
-    __shared__ long long s_q[32], s_r[32];
-    const int lane = static_cast<int>(threadIdx.x);
+// Computed by one of the block's first kInfoWarps warps: each lane forms one
+// quotient and remainder (of a step offset by a period), so the whole set
+// costs the latency of one 64-bit division instead of some twenty in a row.
+// `prev`: first step of the launch before.
+constexpr int kInfoWarps = 4;
+
+__device__ void make_step_info(const InstDev& I, std::int64_t step, std::int64_t prev,
+                               StepInfo& S) {
+    __shared__ long long s_qs[kInfoWarps][32], s_rs[kInfoWarps][32];
+    long long* const s_q = s_qs[threadIdx.x >> 5];
+    long long* const s_r = s_rs[threadIdx.x >> 5];
+    const int lane = static_cast<int>(threadIdx.x & 31u);
     const int P = I.sic_parts;
     std::int64_t n = step, d = I.slots;  // lane 0: ring slot
     if (lane == 1) { n = step - I.d_a2n; d = I.sic_interval; }
-    if (lane == 2) { n = step - I.d_a2n; }
-    if (lane == 3) { n = step - 1 + I.d_e; }
-    if (lane == 4) { n = step - 1 + I.d_i; }
+    if (lane == 2) { n = step - I.d_a2n; d = I.fac_slots; }
+    if (lane == 3) { n = prev + I.d_e; }
+    if (lane == 4) { n = prev + I.d_i; }
     if (lane == 5) { n = step + I.d_e; }
     if (lane == 6) { n = step + I.d_i; }
     if (lane == 7) { d = 3; }
@@ -87,15 +95,18 @@ __device__ void make_step_info(const InstDev& I, std::int64_t step, StepInfo& S)
     if (lane == 12) { d = I.a_steps_per_noise; }
     if (lane >= 13 && lane < 13 + P) { n = step + P - (lane - 13) - I.d_a2n; d = I.sic_interval; }
     if (lane >= 13 + P && lane < 13 + 2 * P) { n = step + P - (lane - 13 - P) - I.d_a2n; }
-    if (lane == 29) { d = I.slots + 1; }
-    if (lane == 30) { n = step + 1; d = I.slots + 1; }
-    if (lane == 31) { n = step - I.d_a2n; d = I.slots + 1; }
+    // (eight parts leave no lane, but then the factors are the arena's)
+    if (lane == 28 && P < 8) { d = I.fac_slots; }
+    if (lane == 29) { d = I.fany_slots; }
+    if (lane == 30) { n = step + I.fany_ahead; d = I.fany_slots; }
+    if (lane == 31) { n = step - I.d_a2n; d = I.fany_slots; }
     std::int64_t q = -1, r = -1;  // -1: negative numerator (not yet due)
     if (n >= 0) {
         const auto un = static_cast<unsigned long long>(n), ud = static_cast<unsigned long long>(d);
         q = static_cast<std::int64_t>(un / ud);
         r = static_cast<std::int64_t>(un - static_cast<unsigned long long>(q) * ud);
     }
+    __syncwarp();
     s_q[lane] = q;
     s_r[lane] = r;
     __syncwarp();
@@ -104,6 +115,7 @@ __device__ void make_step_info(const InstDev& I, std::int64_t step, StepInfo& S)
         S.slot = static_cast<std::uint32_t>(s_r[0]);
         S.sic_now = s_r[1] == 0;
         S.fslot = s_r[2] >= 0 ? static_cast<std::uint32_t>(s_r[2]) : 0u;
+        S.eslot = static_cast<std::uint32_t>(P < 8 ? s_r[28] : s_r[0]);
         S.sic_due = 0;
         for (int p = 0; p < P; ++p) {
             const bool due = s_r[13 + p] == 0;
@@ -133,6 +145,40 @@ __device__ void make_step_info(const InstDev& I, std::int64_t step, StepInfo& S)
         S.fany_next = static_cast<std::int32_t>(s_r[30]);
         S.fany_read = static_cast<std::int32_t>(s_r[31]);
     }
+}
+
+// The step arithmetic of a launch: its steps and the one after them.
+__device__ void make_span_info(const InstDev& I, const Span& sp, StepInfo* S) {
+    const int warps = min(static_cast<int>(blockDim.x >> 5), kInfoWarps);
+    const int w = static_cast<int>(threadIdx.x >> 5);
+    if (w < warps)
+        for (int j = w; j <= sp.cnt; j += warps)
+            make_step_info(I, I.step0 + sp.k + j, I.step0 + sp.kprev, S[j]);
+}
+
+// Steps of the launch that this instance still runs.
+__device__ __forceinline__ int span_count(const InstDev& I, std::int64_t first, int cnt) {
+    const std::int64_t left = I.end_step - first;
+    return left < cnt ? static_cast<int>(left) : cnt;
+}
+
+// A spike list: its header word and its records.
+struct SpikeList {
+    unsigned long long* packed;
+    std::uint32_t* meta;
+    double* val;
+};
+
+// List `id` (see Span): 3 the arena's list `ls`, else span header id with the
+// records of launch index i.
+template <bool kSpan>
+__device__ __forceinline__ SpikeList spike_list(const InstDev& I, int id, std::uint32_t ls, int i) {
+    if (!kSpan || id == 3) {
+        const std::size_t o = static_cast<std::size_t>(ls) * I.N;
+        return SpikeList{I.spk_packed + ls * kHeaderStride, I.spk_meta + 4 * o, I.spk_val + 2 * o};
+    }
+    const std::size_t o = static_cast<std::size_t>(i & 1) * I.span_cap;
+    return SpikeList{I.span_packed + id * kHeaderStride, I.span_meta + 4 * o, I.span_val + 2 * o};
 }
 
 // Routes one arrival the way NeuronPopulation::add_synaptic_input does
@@ -465,7 +511,7 @@ __device__ __forceinline__ void sic_prefetch(const InstDev& I, std::uint32_t t, 
         e[k] = static_cast<std::uint32_t>(k) < len ? __ldg(I.sic_ent + o0 + k * 32) : 0u;
 }
 
-// SIC of a neuron summed by its own thread (fused mode, SIC delay of one step).
+// SIC of a neuron summed by its own thread (fused form).
 __device__ __noinline__ double fused_sic(const InstDev& I, std::uint32_t c, std::uint32_t fslot) {
     std::uint32_t o0, len, e[kSicBatch];
     sic_prefetch(I, c, o0, len, e);
@@ -473,6 +519,62 @@ __device__ __noinline__ double fused_sic(const InstDev& I, std::uint32_t c, std:
     const double v = sic_sum(I, o0, len, e, fslot, 0.0, edges);
     if (edges) atomicAdd(I.counters + 1, edges);
     return v;
+}
+
+// SIC sums of target c by its own thread for the arrival steps S[0], S[1], ...
+// named in `mask`, side by side: each list entry's factors at the arrivals'
+// emission steps are loaded together and its m additions advance the sums as
+// independent chains, each the sequential sum of sic_sum (a zero factor adds
+// +0.0, exact since a sum that starts at +0.0 and adds nonzero values is never
+// -0.0).  The sums go to out[j * stride]; returns the edges summed.
+__device__ __noinline__ unsigned long long sic_span(const InstDev& I, std::uint32_t c,
+                                                    const StepInfo* S, unsigned mask, double* out,
+                                                    unsigned stride) {
+    std::uint32_t o0, len, e[kSicBatch];
+    sic_prefetch(I, c, o0, len, e);
+    double acc[kMaxSpan];
+    std::uint32_t row[kMaxSpan];
+    unsigned long long edges = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxSpan; ++j) {
+        acc[j] = 0.0;
+        row[j] = (mask >> j) & 1u ? S[j].fslot : 0u;
+    }
+    for (std::uint32_t b0 = 0;; b0 += kSicBatch) {
+        bool done = false;
+        for (int q = 0; q < kSicBatch; ++q) {
+            const std::uint32_t m = e[q] & 0xFFu;
+            if (m == 0) {
+                done = true;  // padding ends the list
+                break;
+            }
+            double f[kMaxSpan];
+#pragma unroll
+            for (int j = 0; j < kMaxSpan; ++j)
+                f[j] = (mask >> j) & 1u
+                           ? __ldcg(I.fac + static_cast<std::size_t>(row[j]) * I.NA + (e[q] >> 8))
+                           : 0.0;
+#pragma unroll
+            for (int j = 0; j < kMaxSpan; ++j) {
+                if (f[j] != 0.0) edges += m;
+                f[j] = f[j] == 0.0 ? 0.0 : I.w_a2n * f[j];
+            }
+            for (std::uint32_t r = 0; r < m; ++r) {
+#pragma unroll
+                for (int j = 0; j < kMaxSpan; ++j) acc[j] += f[j];
+            }
+        }
+        if (done || b0 + kSicBatch >= len) break;
+#pragma unroll
+        for (int q = 0; q < kSicBatch; ++q) {
+            const std::uint32_t j = b0 + kSicBatch + q;
+            e[q] = j < len ? __ldg(I.sic_ent + o0 + j * 32) : 0u;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxSpan; ++j)
+        if ((mask >> j) & 1u) out[j * stride] = acc[j];
+    return edges;
 }
 
 // ---------------------------------------------------------------- noise
@@ -486,6 +588,15 @@ __device__ __noinline__ double normal_first_at(std::uint64_t seed, std::uint64_t
 
 __device__ __noinline__ double normal_clamped_at(std::uint64_t seed, std::uint64_t stream) {
     return normal_clamped(seed, stream);
+}
+
+// The noise draw z of neuron c at the step of T (neuron.cpp:243-248).
+__device__ __forceinline__ double noise_draw(const InstDev& I, const NeuronK& P, const StepInfo& T,
+                                             bool exc, std::uint32_t c) {
+    const std::uint64_t idx = exc ? T.noise_e : T.noise_i;
+    return P.independent_noise
+               ? normal_first_at(I.seed ^ kSaltNeuronNoise, idx * kNoiseStride + c)
+               : normal_first_at(I.seed ^ (exc ? kSaltSharedExc : kSaltSharedInh), idx);
 }
 
 // apply_arrivals (network.cpp:301-338) for one target: both short lists in
@@ -535,22 +646,31 @@ __device__ __noinline__ SynIn arrivals_out_of_line(const InstDev& I, std::uint32
 // few spikes of a small network's step, and the arrival lists stay inline.
 // Either order of the spike records gives the same rings (the arrivals are
 // summed in bit order).
-template <bool kPdl, bool kWide>
-__device__ void neuron_role(const InstDev& I, const StepInfo& S, const Work& wk) {
-    __shared__ std::uint32_t s_spk[kMaxBlock];
-    __shared__ double s_val[2 * kMaxBlock];
+//
+// kSpan: launches of several steps (see Span).  The step loop then carries the
+// state in registers, a step's arrivals are loaded while the step before it
+// runs, and the current formed by the neuron's own thread comes from one pass
+// over its list for all of the launch's steps.
+template <bool kPdl, bool kWide, bool kSpan>
+__device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, const Span& sp,
+                            const Work& wk) {
+    // The push in this block (launches of one step): spiking lanes and the
+    // values they deliver.  Several steps: the block's SIC sums [step][thread].
+    constexpr int kThreads = kWide || kSpan ? 128 : kMaxBlock;
+    __shared__ std::uint32_t s_spk[kSpan ? 1 : kThreads];
+    __shared__ double s_val[kSpan ? kMaxSpan * kThreads : 2 * kThreads];
     __shared__ int s_nspk;
-    if (threadIdx.x == 0) s_nspk = 0;
+    if (!kSpan && threadIdx.x == 0) s_nspk = 0;
 
     const std::uint32_t c = wk.first + threadIdx.x;
     const bool active = threadIdx.x < wk.count;
     const bool exc = c < I.NE;
     // Written before the chunk started: read before waiting on the
-    // previous step.
+    // previous launch.
     double Vr = 0.0, bc = 0.0;
     std::uint32_t r0 = 0, len0 = 0, len1 = 0;  // out-edge rows (the wide form: on a spike)
     if (active) {
-        if (!kWide) {  // the wide form reads these where a reset needs them
+        if (!kWide) {  // the wide form reads these where a spike or reset needs them
             Vr = I.V_reset[c];
             bc = I.b[c];
             if (exc) {
@@ -563,29 +683,66 @@ __device__ void neuron_role(const InstDev& I, const StepInfo& S, const Work& wk)
             }
         }
     }
+    const NeuronK& P = exc ? I.pe : I.pi;
+    const std::int64_t first = S[0].step;
+    const int cnt = kSpan ? span_count(I, first, sp.cnt) : (first < I.end_step ? 1 : 0);
+    // The random draws need no memory.  The latency form makes a launch's
+    // Poisson draws and its first noise draw here, beside the launch before:
+    // in the step loop they cost 1,343 of 5,350 cycles per use_case step.
+    // (Counts are held in 8 bits each; 255 and more are drawn again.)
+    constexpr bool kEarlyDraws = kSpan && !kWide;
+    unsigned long long events = 0;
+    int fresh_at = cnt;
+    double z_fresh = 0.0;
+    if (kEarlyDraws && active) {
+        if (P.poiss_rate > 0.0)
+            for (int j = 0; j < cnt; ++j) {
+                Draws r(I.seed ^ kSaltNeuronPoisson,
+                        static_cast<std::uint64_t>(first + j) * kStreamStride + c);
+                const int ev = r.poisson(P.lambda, P.knuth_limit);
+                events |= static_cast<unsigned long long>(min(ev, 255)) << (8 * j);
+            }
+        if (P.noise_std > 0.0) {
+            for (fresh_at = 0; fresh_at < cnt; ++fresh_at)
+                if (exc ? S[fresh_at].fresh_e : S[fresh_at].fresh_i) break;
+            if (fresh_at < cnt) z_fresh = P.noise_std * noise_draw(I, P, S[fresh_at], exc, c);
+        }
+    }
     if (kPdl) grid_dep_wait();
     __syncthreads();
-    const std::int64_t step = S.step;
-    if (step >= I.end_step) return;
+    if (cnt <= 0) return;
+
+    // Steps of the launch whose SIC has emitting astrocytes: the one arriving
+    // at the step (fused) or at the step after it (inline).
+    const int ahead = kSpan && I.sic_inline ? 1 : 0;
+    unsigned sic_mask = 0;
+    if (kSpan && (I.sic_inline || I.fused_sic)) {
+        const int l = static_cast<int>(threadIdx.x & 31u);
+        bool on = false;
+        if (l < cnt) {
+            const StepInfo& T = S[l + ahead];
+            on = T.sic_now && T.fany_read >= 0 && __ldcg(I.fac_any + T.fany_read) != 0u;
+        }
+        sic_mask = __ballot_sync(0xFFFFFFFFu, on);
+    }
 
     if (active) {
-        const NeuronK& P = exc ? I.pe : I.pi;
-        const std::uint32_t slot = S.slot;
-
-        // Every input of the step in one batch of independent loads.
-        const std::size_t ts_ex = static_cast<std::size_t>(slot) * I.ring_ex.n_targets + c;
-        const std::size_t ts_in = static_cast<std::size_t>(slot) * I.ring_in.n_targets + c;
-        const std::uint32_t n_ex = __ldcg(I.ring_ex.cnt + ts_ex);
-        const std::uint32_t n_in = __ldcg(I.ring_in.cnt + ts_in);
+        // Every input of the first step in one batch of independent loads; a
+        // later step's arrivals are loaded while the step before it runs.
+        std::size_t ts_ex = static_cast<std::size_t>(S[0].slot) * I.ring_ex.n_targets + c;
+        std::size_t ts_in = static_cast<std::size_t>(S[0].slot) * I.ring_in.n_targets + c;
+        std::uint32_t n_ex = __ldcg(I.ring_ex.cnt + ts_ex);
+        std::uint32_t n_in = __ldcg(I.ring_in.cnt + ts_in);
         // The first excitatory list value, loaded before the count is known:
         // with a single arrival (the common case) the sum needs no second
         // round trip.
-        const double v0_ex = __ldcg(I.ring_ex.lval + ts_ex * kListCap);
-        const bool sic_due = S.sic_now != 0;
-        double Isic = (sic_due && !I.fused_sic)
-                          ? __ldcg(I.sic_val +
-                                   static_cast<std::size_t>(step & (I.sic_ring - 1)) * I.N + c)
-                          : I.Isic[c];
+        double v0_ex = __ldcg(I.ring_ex.lval + ts_ex * kListCap);
+        // The SIC arriving at the first step; inline, also each later one,
+        // formed during the step before it.
+        const bool sic_load = S[0].sic_now && !I.fused_sic;
+        double sic_next = sic_load ? __ldcg(I.sic_val + static_cast<std::size_t>(first & (I.sic_ring - 1)) * I.N + c)
+                                   : I.Isic[c];
+        double Isic = kSpan && sic_load ? 0.0 : sic_next;
         double V = I.V[c], w = I.w[c], gex = I.gex[c], gin = I.gin[c];
         double dgex = I.dgex[c], dgin = I.dgin[c];
         int refr = I.refr[c];
@@ -599,285 +756,322 @@ __device__ void neuron_role(const InstDev& I, const StepInfo& S, const Work& wk)
             su = I.stp_u[c];
             st = I.stp_t[c];
         }
-
-        // Draws need no memory: they overlap the loads above.
-        int ev = 0;
-        if (P.poiss_rate > 0.0) {
-            Draws r(I.seed ^ kSaltNeuronPoisson,
-                    static_cast<std::uint64_t>(step) * kStreamStride + c);
-            ev = r.poisson(P.lambda, P.knuth_limit);
-        }
         // Noise term noise_std * z (neuron.cpp:243-248), z drawn once per
         // noise interval.
         double zterm = 0.0;
-        if (P.noise_std > 0.0) {
-            if (exc ? S.fresh_e : S.fresh_i) {
-                const std::uint64_t idx = exc ? S.noise_e : S.noise_i;
-                const double z =
-                    P.independent_noise
-                        ? normal_first_at(I.seed ^ kSaltNeuronNoise, idx * kNoiseStride + c)
-                        : normal_first_at(I.seed ^ (exc ? kSaltSharedExc : kSaltSharedInh), idx);
-                zterm = P.noise_std * z;
-                I.noise_n[c] = zterm;
-            } else {
-                zterm = I.noise_n[c];
-            }
-        }
-
-        double exc_in = 0.0, inh_in = 0.0;
-        if constexpr (kWide) {
-            // Most targets of a large network see no arrival or a single
-            // excitatory one in a step; the rest go out of line, so the list
-            // registers are not live on the common path.
-            if (n_ex > 1 || n_in != 0u) {
-                const SynIn a = arrivals_out_of_line(I, slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex);
-                exc_in = a.exc;
-                inh_in = a.inh;
-            } else if (n_ex) {
-                I.ring_ex.cnt[ts_ex] = 0;
-                const double ex = 0.0 + v0_ex;
-                if (ex != 0.0) add_syn(ex, exc_in, inh_in);
-            }
-        } else {
-            apply_arrivals(I, slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex, exc_in, inh_in);
-        }
-        if (sic_due) {
-            if (I.fused_sic)
-                Isic = (S.fany_read >= 0 && __ldcg(I.fac_any + S.fany_read) != 0u)
-                           ? fused_sic(I, c, S.fslot)
-                           : 0.0;  // no emitting astrocyte: the sum of no terms
-            I.Isic[c] = Isic;
-        }
-
-        // Poisson drive and noise (neuron.cpp:228-248)
-        if (ev > 0) exc_in += P.poiss_weight * static_cast<double>(ev);
-        double Iext = Isic;
-        if (P.noise_std > 0.0) Iext += 0.0 + zterm;
-
-        if (exc_in != 0.0) dgex += exc_in * P.psc_ex;
-        if (inh_in != 0.0) dgin += inh_in * P.psc_in;
-
-        const double h = I.ak.h;  // h_step is shared by both models
-        const double half_h = I.ak.half_h, h6 = I.ak.h6;
-        bool spiked = false;
-        for (int s = 0; s < I.ak.substeps; ++s) {
-            const double gex1 = P.decay_ex * (gex + h * dgex);
-            const double dgex1 = P.decay_ex * dgex;
-            const double gin1 = P.decay_in * (gin + h * dgin);
-            const double dgin1 = P.decay_in * dgin;
-            if (refr > 0) {
-                V = kWide ? I.V_reset[c] : Vr;
-                const AdexRates r = adex<false>(P, V, w, gex, gin, Iext);
-                w += h * r.w;
-            } else {
-                // RK4 with the conductances at the start, midpoint and end of
-                // the substep (neuron.cpp:285-298), the four stages unrolled
-                // (no stage selects at run time); the stage sum
-                // k1 + 2 k2 + 2 k3 + k4 accumulates left to right.
-                const double gexm = 0.5 * (gex + gex1), ginm = 0.5 * (gin + gin1);
-                double sV = 0.0, sw = 0.0, xV = V, xw = w;
-#pragma unroll
-                for (int stg = 0; stg < 4; ++stg) {
-                    const double ge = stg == 0 ? gex : (stg < 3 ? gexm : gex1);
-                    const double gi = stg == 0 ? gin : (stg < 3 ? ginm : gin1);
-                    const AdexRates r = adex<true>(P, xV, xw, ge, gi, Iext);
-                    if (stg == 0) {
-                        sV = r.V;
-                        sw = r.w;
-                    } else if (stg < 3) {
-                        sV = fma(2.0, r.V, sV);  // = sV + 2.0 * r.V: 2r is exact
-                        sw = fma(2.0, r.w, sw);
-                    } else {
-                        sV = sV + r.V;
-                        sw = sw + r.w;
-                    }
-                    const double stp = stg < 2 ? half_h : h;
-                    xV = V + stp * r.V;
-                    xw = w + stp * r.w;
-                }
-                V += h6 * sV;
-                w += h6 * sw;
-            }
-            gex = gex1;
-            dgex = dgex1;
-            gin = gin1;
-            dgin = dgin1;
-            if (refr > 0) {
-                --refr;
-            } else if (V >= P.V_peak) {
-                V = kWide ? I.V_reset[c] : Vr;
-                w += kWide ? I.b[c] : bc;
-                refr = P.ref_steps;
-                spiked = true;
-            }
-        }
-        I.V[c] = V;
-        I.w[c] = w;
-        I.gex[c] = gex;
-        I.dgex[c] = dgex;
-        I.gin[c] = gin;
-        I.dgin[c] = dgin;
-        I.refr[c] = refr;
-
-        double v0 = 0.0, v1 = 0.0;  // the values a spike's edges deliver
-        std::uint32_t r1 = 0;
-        if (spiked) {
-            if (kWide) {
-                if (I.stp_on) {
-                    sx = I.stp_x[c];
-                    su = I.stp_u[c];
-                    st = I.stp_t[c];
-                }
-                if (exc) {
-                    r0 = I.exc_rs[c];
-                    len0 = I.exc_rs[c + 1] - r0;
-                    len1 = I.n2a_rs[c + 1] - I.n2a_rs[c];
-                } else {
-                    r0 = I.inh_rs[c - I.NE];
-                    len0 = I.inh_rs[c - I.NE + 1] - r0;
-                }
-            }
-            // Tsodyks-Markram update of this source (network.cpp:230-247); the
-            // value its edges deliver is w*x*u per set.
-            double x = 1.0, u = 1.0;
-            if (I.stp_on) {
-                const double t_now = static_cast<double>(step) * I.dt;
-                const double d = t_now - st;
-                const double xd = exp(div_by(-d, I.tau_rec, I.inv_tau_rec));
-                const double ud =
-                    I.tau_fac < 1e-10 ? 0.0 : exp(div_by(-d, I.tau_fac, I.inv_tau_fac));
-                x = 1.0 + (sx - sx * su - 1.0) * xd;
-                u = I.U + su * (1.0 - I.U) * ud;
-                I.stp_x[c] = x;
-                I.stp_u[c] = u;
-                I.stp_t[c] = t_now;
-            }
-            v0 = exc ? (I.stp_on ? I.w_e * x * u : I.w_e) : (I.stp_on ? I.w_i * x * u : I.w_i);
-            v1 = exc ? (I.stp_on ? I.w_n2a * x * u : I.w_n2a) : 0.0;
-            // n2a row start of an excitatory source (~0: inhibitory), loaded
-            // while the warp's append is formed
-            if (I.deferred_push) r1 = exc ? __ldg(I.n2a_rs + c) : kNoBit;
-            if (!I.deferred_push) {
-                s_val[threadIdx.x * 2 + 0] = v0;
-                s_val[threadIdx.x * 2 + 1] = v1;
-                const int pos = atomicAdd(&s_nspk, 1);
-                s_spk[pos] = threadIdx.x;
-            }
-        }
-
-        if constexpr (!kWide) {
-            if (spiked) {
-                // One atomic reserves this spike's record and edge range.
-                if (I.deferred_push) {
-                    const unsigned long long old = atomicAdd(
-                        I.spk_packed + S.ls * kHeaderStride,
-                        (1ull << 40) | static_cast<unsigned long long>(len0 + len1));
-                    const std::size_t o = static_cast<std::size_t>(S.ls) * I.N + (old >> 40);
-                    *reinterpret_cast<uint4*>(I.spk_meta + 4 * o) = make_uint4(
-                        r1, static_cast<std::uint32_t>(old & 0xFFFFFFFFFFull), r0, len0);
-                    *reinterpret_cast<double2*>(I.spk_val + 2 * o) = make_double2(v0, v1);
-                }
-                if (I.rec_spikes && step >= I.rec_from) {
-                    const unsigned long long li = atomicAdd(I.spike_log_n, 1ULL);
-                    if (li < I.spike_log_cap) {
-                        I.spike_log[li] = (static_cast<unsigned long long>(step) << 32) | c;
-                    } else {
-                        atomicAdd(I.counters + 3, 1ULL);
-                    }
-                }
-                atomicAdd(I.counters + 0, static_cast<unsigned long long>(len0 + len1));
-                atomicAdd(I.counters + 2, 1ULL);
-            }
-        }
-        // The warp's spikes are compacted with a ballot and prefix sums: one
-        // atomic per warp reserves the spike records and edge range of the
-        // deferred push, one the spike-log entries, one each counter; every
-        // spiking lane writes at its rank among the warp's spiking lanes
-        // (ascending source) and at its exclusive prefix of edge counts.
-        // The active lanes of a warp are a prefix of it (threadIdx.x <
-        // wk.count), all of which reach this point.
-        const unsigned lane = threadIdx.x & 31u;
-        const unsigned wbase = threadIdx.x & ~31u;
-        const unsigned left = wk.count - wbase;  // > 0 for an active lane
-        const unsigned act = left >= 32u ? 0xFFFFFFFFu : ((1u << left) - 1u);
-        const unsigned smask = kWide ? __ballot_sync(act, spiked) : 0u;  // syncs act
-        if (kWide && smask != 0u) {
-            const unsigned rank = __popc(smask & ((1u << lane) - 1u));
-            const int leader = __ffs(smask) - 1;
-            const unsigned nspk = __popc(smask);
+        if (kSpan && P.noise_std > 0.0 && !(exc ? S[0].fresh_e : S[0].fresh_i)) zterm = I.noise_n[c];
+        bool sic_set = false;
+        if (kSpan && sic_mask != 0u) {
             const unsigned long long edges =
-                spiked ? static_cast<unsigned long long>(len0 + len1) : 0ull;
-            unsigned long long incl = edges;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned long long t = __shfl_up_sync(act, incl, d);
-                if (lane >= static_cast<unsigned>(d)) incl += t;
-            }
-            const int last = 31 - __clz(act);
-            const unsigned long long total = __shfl_sync(act, incl, last);
-            unsigned long long base_spk = 0, base_log = 0;
-            const bool logging = I.rec_spikes && step >= I.rec_from;
-            if (lane == static_cast<unsigned>(leader)) {
-                if (I.deferred_push)
-                    base_spk = atomicAdd(I.spk_packed + S.ls * kHeaderStride,
-                                         (static_cast<unsigned long long>(nspk) << 40) | total);
-                if (logging) base_log = atomicAdd(I.spike_log_n, static_cast<unsigned long long>(nspk));
-                atomicAdd(I.counters + 0, total);
-                atomicAdd(I.counters + 2, static_cast<unsigned long long>(nspk));
-            }
-            base_spk = __shfl_sync(act, base_spk, leader);
-            base_log = __shfl_sync(act, base_log, leader);
-            if (spiked) {
-                if (I.deferred_push) {
-                    const std::size_t o = static_cast<std::size_t>(S.ls) * I.N + (base_spk >> 40) + rank;
-                    const unsigned long long eoff = (base_spk & 0xFFFFFFFFFFull) + (incl - edges);
-                    *reinterpret_cast<uint4*>(I.spk_meta + 4 * o) =
-                        make_uint4(r1, static_cast<std::uint32_t>(eoff), r0, len0);
-                    *reinterpret_cast<double2*>(I.spk_val + 2 * o) = make_double2(v0, v1);
+                sic_span(I, c, S + ahead, sic_mask, s_val + threadIdx.x, kThreads);
+            if (edges) atomicAdd(I.counters + 1, edges);
+        }
+        // The sum formed for step `at` (fused: its own, inline: the next one's);
+        // without an emitting astrocyte the sum of no terms.
+        const auto own_sic = [&](int at) {
+            if (kSpan) return (sic_mask >> at) & 1u ? s_val[at * kThreads + threadIdx.x] : 0.0;
+            return S[0].fany_read >= 0 && __ldcg(I.fac_any + S[0].fany_read) != 0u
+                       ? fused_sic(I, c, S[0].fslot)
+                       : 0.0;
+        };
+
+        const auto store_state = [&] {
+            I.V[c] = V;
+            I.w[c] = w;
+            I.gex[c] = gex;
+            I.dgex[c] = dgex;
+            I.gin[c] = gin;
+            I.dgin[c] = dgin;
+            I.refr[c] = refr;
+        };
+
+        const int n_steps = kSpan ? cnt : 1;
+        for (int j = 0; j < n_steps; ++j) {
+            const StepInfo& T = S[j];
+            const std::int64_t step = first + j;
+            int ev = kEarlyDraws ? static_cast<int>((events >> (8 * j)) & 0xFFu) : 255;
+            if (ev == 255) {
+                ev = 0;
+                if (P.poiss_rate > 0.0) {
+                    Draws r(I.seed ^ kSaltNeuronPoisson,
+                            static_cast<std::uint64_t>(step) * kStreamStride + c);
+                    ev = r.poisson(P.lambda, P.knuth_limit);
                 }
-                if (logging) {
-                    const unsigned long long li = base_log + rank;
-                    if (li < I.spike_log_cap) {
-                        I.spike_log[li] = (static_cast<unsigned long long>(step) << 32) | c;
+            }
+            if (!kSpan && P.noise_std > 0.0 && !(exc ? T.fresh_e : T.fresh_i)) zterm = I.noise_n[c];
+            if (P.noise_std > 0.0 && (exc ? T.fresh_e : T.fresh_i)) {
+                zterm = kEarlyDraws && j == fresh_at ? z_fresh
+                                                : P.noise_std * noise_draw(I, P, T, exc, c);
+                I.noise_n[c] = zterm;
+            }
+
+            double exc_in = 0.0, inh_in = 0.0;
+            if constexpr (kWide || kSpan) {
+                // Most targets see no arrival or a single excitatory one in a
+                // step; the rest go out of line, so the list registers are not
+                // live on the common path.
+                if (n_ex > 1 || n_in != 0u) {
+                    const SynIn a = arrivals_out_of_line(I, T.slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex);
+                    exc_in = a.exc;
+                    inh_in = a.inh;
+                } else if (n_ex) {
+                    I.ring_ex.cnt[ts_ex] = 0;
+                    const double ex = 0.0 + v0_ex;
+                    if (ex != 0.0) add_syn(ex, exc_in, inh_in);
+                }
+            } else {
+                apply_arrivals(I, T.slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex, exc_in, inh_in);
+            }
+            if (T.sic_now) {
+                Isic = I.fused_sic ? own_sic(j) : sic_next;
+                sic_set = true;
+                if (!kSpan) I.Isic[c] = Isic;
+            }
+            if (kSpan && j + 1 < cnt) {
+                ts_ex = static_cast<std::size_t>(S[j + 1].slot) * I.ring_ex.n_targets + c;
+                ts_in = static_cast<std::size_t>(S[j + 1].slot) * I.ring_in.n_targets + c;
+                n_ex = __ldcg(I.ring_ex.cnt + ts_ex);
+                n_in = __ldcg(I.ring_in.cnt + ts_in);
+                v0_ex = __ldcg(I.ring_ex.lval + ts_ex * kListCap);
+                if (I.sic_side && S[j + 1].sic_now)
+                    sic_next = __ldcg(I.sic_val + static_cast<std::size_t>((step + 1) & (I.sic_ring - 1)) * I.N + c);
+            }
+            if (kSpan && I.sic_inline && S[j + 1].sic_now) {
+                sic_next = own_sic(j);
+                if (j + 1 == cnt)
+                    I.sic_val[static_cast<std::size_t>((step + 1) & (I.sic_ring - 1)) * I.N + c] = sic_next;
+            }
+
+            // Poisson drive and noise (neuron.cpp:228-248)
+            if (ev > 0) exc_in += P.poiss_weight * static_cast<double>(ev);
+            double Iext = Isic;
+            if (P.noise_std > 0.0) Iext += 0.0 + zterm;
+
+            if (exc_in != 0.0) dgex += exc_in * P.psc_ex;
+            if (inh_in != 0.0) dgin += inh_in * P.psc_in;
+
+            const double h = I.ak.h;  // h_step is shared by both models
+            const double half_h = I.ak.half_h, h6 = I.ak.h6;
+            bool spiked = false;
+            for (int s = 0; s < I.ak.substeps; ++s) {
+                const double gex1 = P.decay_ex * (gex + h * dgex);
+                const double dgex1 = P.decay_ex * dgex;
+                const double gin1 = P.decay_in * (gin + h * dgin);
+                const double dgin1 = P.decay_in * dgin;
+                if (refr > 0) {
+                    V = kWide ? I.V_reset[c] : Vr;
+                    const AdexRates r = adex<false>(P, V, w, gex, gin, Iext);
+                    w += h * r.w;
+                } else {
+                    // RK4 with the conductances at the start, midpoint and end of
+                    // the substep (neuron.cpp:285-298), the four stages unrolled
+                    // (no stage selects at run time); the stage sum
+                    // k1 + 2 k2 + 2 k3 + k4 accumulates left to right.
+                    const double gexm = 0.5 * (gex + gex1), ginm = 0.5 * (gin + gin1);
+                    double sV = 0.0, sw = 0.0, xV = V, xw = w;
+    #pragma unroll
+                    for (int stg = 0; stg < 4; ++stg) {
+                        const double ge = stg == 0 ? gex : (stg < 3 ? gexm : gex1);
+                        const double gi = stg == 0 ? gin : (stg < 3 ? ginm : gin1);
+                        const AdexRates r = adex<true>(P, xV, xw, ge, gi, Iext);
+                        if (stg == 0) {
+                            sV = r.V;
+                            sw = r.w;
+                        } else if (stg < 3) {
+                            sV = fma(2.0, r.V, sV);  // = sV + 2.0 * r.V: 2r is exact
+                            sw = fma(2.0, r.w, sw);
+                        } else {
+                            sV = sV + r.V;
+                            sw = sw + r.w;
+                        }
+                        const double stp = stg < 2 ? half_h : h;
+                        xV = V + stp * r.V;
+                        xw = w + stp * r.w;
+                    }
+                    V += h6 * sV;
+                    w += h6 * sw;
+                }
+                gex = gex1;
+                dgex = dgex1;
+                gin = gin1;
+                dgin = dgin1;
+                if (refr > 0) {
+                    --refr;
+                } else if (V >= P.V_peak) {
+                    V = kWide ? I.V_reset[c] : Vr;
+                    w += kWide ? I.b[c] : bc;
+                    refr = P.ref_steps;
+                    spiked = true;
+                }
+            }
+            if (!kSpan) store_state();  // on its way before the spike's work
+            double v0 = 0.0, v1 = 0.0;  // the values a spike's edges deliver
+            std::uint32_t r1 = 0;
+            if (__builtin_expect(spiked, 0)) {
+                if (kWide) {
+                    if (I.stp_on) {
+                        sx = I.stp_x[c];
+                        su = I.stp_u[c];
+                        st = I.stp_t[c];
+                    }
+                    if (exc) {
+                        r0 = I.exc_rs[c];
+                        len0 = I.exc_rs[c + 1] - r0;
+                        len1 = I.n2a_rs[c + 1] - I.n2a_rs[c];
                     } else {
-                        atomicAdd(I.counters + 3, 1ULL);
+                        r0 = I.inh_rs[c - I.NE];
+                        len0 = I.inh_rs[c - I.NE + 1] - r0;
+                    }
+                }
+                // Tsodyks-Markram update of this source (network.cpp:230-247); the
+                // value its edges deliver is w*x*u per set.
+                double x = 1.0, u = 1.0;
+                if (I.stp_on) {
+                    const double t_now = static_cast<double>(step) * I.dt;
+                    const double d = t_now - st;
+                    const double xd = exp(div_by(-d, I.tau_rec, I.inv_tau_rec));
+                    const double ud =
+                        I.tau_fac < 1e-10 ? 0.0 : exp(div_by(-d, I.tau_fac, I.inv_tau_fac));
+                    x = 1.0 + (sx - sx * su - 1.0) * xd;
+                    u = I.U + su * (1.0 - I.U) * ud;
+                    I.stp_x[c] = sx = x;
+                    I.stp_u[c] = su = u;
+                    I.stp_t[c] = st = t_now;
+                }
+                v0 = exc ? (I.stp_on ? I.w_e * x * u : I.w_e) : (I.stp_on ? I.w_i * x * u : I.w_i);
+                v1 = exc ? (I.stp_on ? I.w_n2a * x * u : I.w_n2a) : 0.0;
+                // n2a row start of an excitatory source (~0: inhibitory), loaded
+                // while the warp's append is formed
+                if (I.deferred_push) r1 = exc ? __ldg(I.n2a_rs + c) : kNoBit;
+                if (!I.deferred_push) {
+                    s_val[threadIdx.x * 2 + 0] = v0;
+                    s_val[threadIdx.x * 2 + 1] = v1;
+                    const int pos = atomicAdd(&s_nspk, 1);
+                    s_spk[pos] = threadIdx.x;
+                }
+            }
+
+            if constexpr (!kWide) {
+                if (spiked) {
+                    // One atomic reserves this spike's record and edge range.
+                    if (I.deferred_push) {
+                        const SpikeList L = spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i);
+                        const unsigned long long old = atomicAdd(
+                            L.packed, (1ull << 40) | static_cast<unsigned long long>(len0 + len1));
+                        const std::size_t o = old >> 40;
+                        *reinterpret_cast<uint4*>(L.meta + 4 * o) =
+                            make_uint4(r1, static_cast<std::uint32_t>(old & 0xFFFFFFFFFFull), r0,
+                                       kSpan ? len0 | static_cast<std::uint32_t>(j) << 28 : len0);
+                        *reinterpret_cast<double2*>(L.val + 2 * o) = make_double2(v0, v1);
+                    }
+                    if (I.rec_spikes && step >= I.rec_from) {
+                        const unsigned long long li = atomicAdd(I.spike_log_n, 1ULL);
+                        if (li < I.spike_log_cap) {
+                            I.spike_log[li] = (static_cast<unsigned long long>(step) << 32) | c;
+                        } else {
+                            atomicAdd(I.counters + 3, 1ULL);
+                        }
+                    }
+                    atomicAdd(I.counters + 0, static_cast<unsigned long long>(len0 + len1));
+                    atomicAdd(I.counters + 2, 1ULL);
+                }
+            }
+            // The warp's spikes are compacted with a ballot and prefix sums: one
+            // atomic per warp reserves the spike records and edge range of the
+            // deferred push, one the spike-log entries, one each counter; every
+            // spiking lane writes at its rank among the warp's spiking lanes
+            // (ascending source) and at its exclusive prefix of edge counts.
+            // The active lanes of a warp are a prefix of it (threadIdx.x <
+            // wk.count), all of which reach this point.
+            const unsigned lane = threadIdx.x & 31u;
+            const unsigned wbase = threadIdx.x & ~31u;
+            const unsigned left = wk.count - wbase;  // > 0 for an active lane
+            const unsigned act = left >= 32u ? 0xFFFFFFFFu : ((1u << left) - 1u);
+            const unsigned smask = kWide ? __ballot_sync(act, spiked) : 0u;  // syncs act
+            if (kWide && smask != 0u) {
+                const unsigned rank = __popc(smask & ((1u << lane) - 1u));
+                const int leader = __ffs(smask) - 1;
+                const unsigned nspk = __popc(smask);
+                const unsigned long long edges =
+                    spiked ? static_cast<unsigned long long>(len0 + len1) : 0ull;
+                unsigned long long incl = edges;
+    #pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned long long t = __shfl_up_sync(act, incl, d);
+                    if (lane >= static_cast<unsigned>(d)) incl += t;
+                }
+                const int last = 31 - __clz(act);
+                const unsigned long long total = __shfl_sync(act, incl, last);
+                unsigned long long base_spk = 0, base_log = 0;
+                const bool logging = I.rec_spikes && step >= I.rec_from;
+                if (lane == static_cast<unsigned>(leader)) {
+                    if (I.deferred_push)
+                        base_spk = atomicAdd(spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i).packed,
+                                             (static_cast<unsigned long long>(nspk) << 40) | total);
+                    if (logging) base_log = atomicAdd(I.spike_log_n, static_cast<unsigned long long>(nspk));
+                    atomicAdd(I.counters + 0, total);
+                    atomicAdd(I.counters + 2, static_cast<unsigned long long>(nspk));
+                }
+                base_spk = __shfl_sync(act, base_spk, leader);
+                base_log = __shfl_sync(act, base_log, leader);
+                if (spiked) {
+                    if (I.deferred_push) {
+                        const SpikeList L = spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i);
+                        const std::size_t o = (base_spk >> 40) + rank;
+                        const unsigned long long eoff = (base_spk & 0xFFFFFFFFFFull) + (incl - edges);
+                        *reinterpret_cast<uint4*>(L.meta + 4 * o) =
+                            make_uint4(r1, static_cast<std::uint32_t>(eoff), r0,
+                                       kSpan ? len0 | static_cast<std::uint32_t>(j) << 28 : len0);
+                        *reinterpret_cast<double2*>(L.val + 2 * o) = make_double2(v0, v1);
+                    }
+                    if (logging) {
+                        const unsigned long long li = base_log + rank;
+                        if (li < I.spike_log_cap) {
+                            I.spike_log[li] = (static_cast<unsigned long long>(step) << 32) | c;
+                        } else {
+                            atomicAdd(I.counters + 3, 1ULL);
+                        }
                     }
                 }
             }
-        }
 
-        if (I.rec_neuron_max > 0 && c < I.rec_neuron_max && S.rec_now) {
-            const std::size_t row = S.rec_row;
-            I.rec_V[row * I.rec_neuron_max + c] = V;
-            I.rec_Isic[row * I.rec_neuron_max + c] = Isic;
+            if (I.rec_neuron_max > 0 && c < I.rec_neuron_max && T.rec_now) {
+                const std::size_t row = T.rec_row;
+                I.rec_V[row * I.rec_neuron_max + c] = V;
+                I.rec_Isic[row * I.rec_neuron_max + c] = Isic;
+            }
+        }
+        if (kSpan) {
+            store_state();
+            if (sic_set) I.Isic[c] = Isic;
         }
     }
 
     // Push the out-edges of this block's spiking sources into the rings of
     // their arrival steps (deliver_spikes, network.cpp:249-279) when the
-    // push is not deferred to the next step.
-    if (I.deferred_push) return;
+    // push is not deferred (launches of one step).
+    if (kSpan || I.deferred_push) return;
     __syncthreads();
     const int nspk = s_nspk;
     for (int q = 0; q < nspk; ++q) {
         const std::uint32_t lane = s_spk[q];
         const std::uint32_t j = wk.first + lane;
         if (j < I.NE) {
-            push_row(I.exc_rs, I.ring_ex, j, S.now_e, s_val[2 * lane]);
-            push_row(I.n2a_rs, I.ring_as, j, S.now_e, s_val[2 * lane + 1]);
+            push_row(I.exc_rs, I.ring_ex, j, S[0].now_e, s_val[2 * lane]);
+            push_row(I.n2a_rs, I.ring_as, j, S[0].now_e, s_val[2 * lane + 1]);
         } else {
-            push_row(I.inh_rs, I.ring_in, j - I.NE, S.now_i, s_val[2 * lane]);
+            push_row(I.inh_rs, I.ring_in, j - I.NE, S[0].now_i, s_val[2 * lane]);
         }
     }
 }
 
-// Deferred push of the spikes of step-1.  The participating blocks stride
-// over the flat edge space of that step (edge x belongs to the spike whose
+// Deferred push of the spikes of the launch before.  The participating blocks
+// stride over the flat edge space of that launch (edge x belongs to the spike whose
 // range holds it, found by binary search in shared memory), so the work is
 // split evenly whatever the number of spikes.
 constexpr int kPushBatch = 256;
 
-// The deferred push of the spikes of step-1 by participant `rank` of
+// The deferred push of the spikes of list L by participant `rank` of
 // `nranks` (each a block).  The spike list is cut into batches of
 // kPushBatch spikes.  kDealt (the wide form, whose bursts have ~10^4 helper
 // blocks and up to ~60 batches): the participants are dealt over the
@@ -890,18 +1084,18 @@ constexpr int kPushBatch = 256;
 // batches) every participant stages every batch and edge x of the flat edge
 // space goes to thread x % (nranks * blockDim.x); the dealt form measured
 // 0.16 us slower per paper-sparse step there.
-template <bool kDealt>
-__device__ void push_spikes(const InstDev& I, const StepInfo& S, unsigned long long packed,
-                            std::uint32_t rank, std::uint32_t nranks) {
+template <bool kDealt, bool kSpan>
+__device__ void push_spikes(const InstDev& I, const StepInfo& S, const SpikeList& L,
+                            unsigned long long packed, std::uint32_t rank,
+                            std::uint32_t nranks) {
     __shared__ std::uint32_t s_off[kPushBatch + 1], s_r0[kPushBatch], s_len0[kPushBatch],
-        s_r1[kPushBatch];
+        s_r1[kPushBatch], s_slot[kSpan ? kPushBatch : 1];
     __shared__ double s_v[2 * kPushBatch];
     const std::uint32_t n = static_cast<std::uint32_t>(packed >> 40);
     const std::uint32_t total = static_cast<std::uint32_t>(packed & 0xFFFFFFFFFFull);
     if (n == 0) return;  // block-uniform
     const std::uint32_t nbatch = (n + kPushBatch - 1) / kPushBatch;
-    const std::uint32_t as_e = S.push_e, as_i = S.push_i;
-    const std::size_t base = static_cast<std::size_t>(S.ls_prev) * I.N;
+    const std::uint32_t slots = static_cast<std::uint32_t>(I.slots);
     // first batch, rank among the batch's participants, their number (no
     // division in the common single-batch case)
     std::uint32_t first = rank, q = 0, share = 1;
@@ -925,18 +1119,22 @@ __device__ void push_spikes(const InstDev& I, const StepInfo& S, unsigned long l
         const std::uint32_t nb = min(static_cast<std::uint32_t>(kPushBatch), n - b0);
         __syncthreads();
         for (std::uint32_t i = threadIdx.x; i < nb; i += blockDim.x) {
-            const std::size_t o = base + b0 + i;
-            const uint4 m = __ldcg(reinterpret_cast<const uint4*>(I.spk_meta + 4 * o));
-            const double2 v = __ldcg(reinterpret_cast<const double2*>(I.spk_val + 2 * o));
+            const std::size_t o = b0 + i;
+            const uint4 m = __ldcg(reinterpret_cast<const uint4*>(L.meta + 4 * o));
+            const double2 v = __ldcg(reinterpret_cast<const double2*>(L.val + 2 * o));
             s_r1[i] = m.x;  // n2a row start; kNoBit marks an inhibitory source
             s_off[i] = m.y;
             s_r0[i] = m.z;
-            s_len0[i] = m.w;
+            s_len0[i] = kSpan ? m.w & 0x0FFFFFFFu : m.w;
+            if (kSpan) {  // the ring slot of the spike's own step
+                const std::uint32_t at = (m.x == kNoBit ? S.push_i : S.push_e) + (m.w >> 28);
+                s_slot[i] = at < slots ? at : at - slots;
+            }
             s_v[2 * i] = v.x;
             s_v[2 * i + 1] = v.y;
         }
         if (threadIdx.x == 0)
-            s_off[nb] = b0 + nb < n ? __ldcg(I.spk_meta + 4 * (base + b0 + nb) + 1) : total;
+            s_off[nb] = b0 + nb < n ? __ldcg(L.meta + 4 * static_cast<std::size_t>(b0 + nb) + 1) : total;
         __syncthreads();
         // The list order is the atomic order, so offsets ascend along it.
         const std::uint32_t x0 = s_off[0], x1 = s_off[nb];
@@ -948,12 +1146,14 @@ __device__ void push_spikes(const InstDev& I, const StepInfo& S, unsigned long l
             unsigned long long pe[kPushGroup];
             double val[kPushGroup];
             int which[kPushGroup];  // 0 inh, 1 exc, 2 astrocyte, -1 none
+            std::uint32_t slot[kPushGroup];
 #pragma unroll
             for (int u = 0; u < kPushGroup; ++u) {
                 const std::uint32_t x = xg + static_cast<std::uint32_t>(u) * stride;
                 which[u] = -1;
                 pe[u] = 0;
                 val[u] = 0.0;
+                slot[u] = 0;
                 if (x < x1) {
                     std::uint32_t lo = 0, hi = nb;  // last entry with s_off <= x
                     while (hi - lo > 1) {
@@ -961,6 +1161,9 @@ __device__ void push_spikes(const InstDev& I, const StepInfo& S, unsigned long l
                         if (s_off[mid] <= x) lo = mid; else hi = mid;
                     }
                     const std::uint32_t k = x - s_off[lo];
+                    slot[u] = kSpan                ? s_slot[lo]
+                              : s_r1[lo] == kNoBit ? S.push_i
+                                                   : S.push_e;
                     if (s_r1[lo] == kNoBit) {
                         which[u] = 0;
                         pe[u] = __ldg(I.ring_in.edge + s_r0[lo] + k);
@@ -978,9 +1181,9 @@ __device__ void push_spikes(const InstDev& I, const StepInfo& S, unsigned long l
             }
 #pragma unroll
             for (int u = 0; u < kPushGroup; ++u) {
-                if (which[u] == 0) push_edge(I.ring_in, as_i, pe[u], val[u]);
-                else if (which[u] == 1) push_edge(I.ring_ex, as_e, pe[u], val[u]);
-                else if (which[u] == 2) push_edge(I.ring_as, as_e, pe[u], val[u]);
+                if (which[u] == 0) push_edge(I.ring_in, slot[u], pe[u], val[u]);
+                else if (which[u] == 1) push_edge(I.ring_ex, slot[u], pe[u], val[u]);
+                else if (which[u] == 2) push_edge(I.ring_as, slot[u], pe[u], val[u]);
             }
         }
     }
@@ -994,45 +1197,59 @@ __device__ __forceinline__ bool push_burst(const InstDev& I, unsigned long long 
            static_cast<unsigned long long>(kBurstEdgesPerThread) * blockDim.x * I.push_blocks;
 }
 
-// Deferred push of the spikes of step-1 by the PUSH blocks (joined by every
-// other block of the instance in a burst).  One thread also clears the list
-// slot the next step appends to.
-template <bool kPdl, bool kWide>
-__device__ void push_role(const InstDev& I, const StepInfo& S, const Work& wk) {
+// The list this launch pushes has spikes to push.  The arena's list is left
+// alone by an instance that has reached its end (a later chunk pushes it);
+// spikes in a span list are pushed by the next launch whether or not the
+// instance runs on.
+template <bool kSpan>
+__device__ __forceinline__ bool push_pending(const InstDev& I, const StepInfo& S, const Span& sp) {
+    return (kSpan && sp.src != 3) || (S.step > 0 && S.step < I.end_step);
+}
+
+// Deferred push of the spikes of the launch before by the PUSH blocks (joined
+// by every other block of the instance in a burst).  One thread also clears
+// the list header the next launch appends to.
+template <bool kPdl, bool kWide, bool kSpan>
+__device__ void push_role(const InstDev& I, const StepInfo& S, const Span& sp, const Work& wk) {
     if (kPdl) grid_dep_wait();
-    const std::int64_t step = S.step;
-    if (step >= I.end_step) return;
-    if (wk.first == 0 && threadIdx.x == 0) I.spk_packed[S.ls_next * kHeaderStride] = 0;
-    if (step == 0) return;
-    const unsigned long long packed = __ldcg(I.spk_packed + S.ls_prev * kHeaderStride);
+    if (wk.first == 0 && threadIdx.x == 0) {
+        if (kSpan && sp.clear >= 0) I.span_packed[sp.clear * kHeaderStride] = 0;
+        if ((!kSpan || (sp.src == 3 && sp.dst == 3)) && S.step < I.end_step)
+            I.spk_packed[S.ls_next * kHeaderStride] = 0;
+        if (kSpan && sp.clear_arena && I.step0 < I.end_step)
+            for (int l = 0; l < 3; ++l) I.spk_packed[l * kHeaderStride] = 0;
+    }
+    if (!push_pending<kSpan>(I, S, sp)) return;
+    const SpikeList L = spike_list<kSpan>(I, sp.src, S.ls_prev, sp.i - 1);
+    const unsigned long long packed = __ldcg(L.packed);
     const std::uint32_t nranks = static_cast<std::uint32_t>(I.push_blocks) +
                                  (push_burst(I, packed) ? I.push_helpers : 0u);
-    push_spikes<kWide>(I, S, packed, wk.first, nranks);
+    push_spikes<kWide, kSpan>(I, S, L, packed, wk.first, nranks);
 }
 
-// A non-push block's share of a burst push, after its own role.
 // A non-push block's share of a burst push (its rank among the helpers).
-template <bool kWide>
+template <bool kWide, bool kSpan>
 __device__ __noinline__ void help_push_spikes(const InstDev& I, const StepInfo& S,
-                                              unsigned long long packed, std::uint32_t helper) {
-    push_spikes<kWide>(I, S, packed, static_cast<std::uint32_t>(I.push_blocks) + helper,
-                static_cast<std::uint32_t>(I.push_blocks + I.push_helpers));
+                                              const SpikeList& L, unsigned long long packed,
+                                              std::uint32_t helper) {
+    push_spikes<kWide, kSpan>(I, S, L, packed, static_cast<std::uint32_t>(I.push_blocks) + helper,
+                       static_cast<std::uint32_t>(I.push_blocks + I.push_helpers));
 }
 
-// After its own role, a block joins the push of step-1's spikes when that
-// push is a burst.  `burst` carries the answer across the items a block runs
-// in one step of one instance (-1: not known yet, else 0 or 1), so the spike
-// count is read once per block rather than once per item; the new answer is
-// returned.  Only a burst leaves the inline path.
-template <bool kWide>
-__device__ __forceinline__ int help_push(const InstDev& I, const StepInfo& S, const Work& wk,
-                                         int burst) {
-    if (burst == 0 || !I.deferred_push || wk.helper == kNoHelper || S.step == 0 ||
-        S.step >= I.end_step)
+// After its own role, a block joins the push of the spikes of the launch
+// before when that push is a burst.  `burst` carries the answer across the
+// items a block runs in one launch of one instance (-1: not known yet, else 0
+// or 1), so the spike count is read once per block rather than once per item;
+// the new answer is returned.  Only a burst leaves the inline path.
+template <bool kWide, bool kSpan>
+__device__ __forceinline__ int help_push(const InstDev& I, const StepInfo& S, const Span& sp,
+                                         const Work& wk, int burst) {
+    if (burst == 0 || !I.deferred_push || wk.helper == kNoHelper || !push_pending<kSpan>(I, S, sp))
         return burst;
-    const unsigned long long packed = __ldcg(I.spk_packed + S.ls_prev * kHeaderStride);
+    const SpikeList L = spike_list<kSpan>(I, sp.src, S.ls_prev, sp.i - 1);
+    const unsigned long long packed = __ldcg(L.packed);
     if (!push_burst(I, packed)) return 0;
-    help_push_spikes<kWide>(I, S, packed, wk.helper);
+    help_push_spikes<kWide, kSpan>(I, S, L, packed, wk.helper);
     return 1;
 }
 
@@ -1052,8 +1269,16 @@ __device__ __noinline__ void astro_update_f32(const InstDev& I, double ca_tot, d
     hh = hv;
 }
 
-template <bool kPdl, bool kF32>
-__device__ void astro_role(const InstDev& I, const StepInfo& S, const Work& wk) {
+// The noise draw z of astrocyte a at the step of T (astrocyte.cpp:307-329).
+__device__ __forceinline__ double astro_noise_draw(const InstDev& I, const StepInfo& T,
+                                                   std::uint32_t a) {
+    return normal_clamped_at(I.seed ^ kSaltAstroNoise,
+                             I.a_indep ? T.noise_a * kStreamStride + a : T.noise_a);
+}
+
+template <bool kPdl, bool kF32, bool kWide, bool kSpan>
+__device__ void astro_role(const InstDev& I, const StepInfo* __restrict__ S, const Span& sp,
+                           const Work& wk) {
     const std::uint32_t a = wk.first + threadIdx.x;
     const bool active = threadIdx.x < wk.count;
     double ca_tot = I.Ca_tot_u, ip3_0 = I.IP3_0_u, tau = I.tau_u, inv_tau = I.inv_tau_u,
@@ -1065,64 +1290,95 @@ __device__ void astro_role(const InstDev& I, const StepInfo& S, const Work& wk) 
         inv_tau = I.inv_tau[a];
         delta = I.delta[a];
     }
-    if (kPdl) grid_dep_wait();
-    const std::int64_t step = S.step;
-    // The next step's emission flag starts clear (nothing reads or writes
-    // that entry during this step: see InstDev::fac_any).
-    if (wk.first == 0 && threadIdx.x == 0 && step < I.end_step) I.fac_any[S.fany_next] = 0u;
-    if (!active || step >= I.end_step) return;
-    const std::uint32_t slot = S.slot;
-    const std::size_t ts = static_cast<std::size_t>(slot) * I.ring_as.n_targets + a;
-    const std::uint32_t n = __ldcg(I.ring_as.cnt + ts);
-    double ca = I.Ca[a], ip3 = I.IP3[a], hh = I.h[a];
-    // drive_astrocytes (network.cpp:340-355) and the noise draw
-    // (astrocyte.cpp:307-329): no memory, overlapping the loads.
-    int ev = 0;
-    if (I.a_rate > 0.0) {
-        Draws r(I.seed ^ kSaltAstroPoisson, static_cast<std::uint64_t>(step) * kStreamStride + a);
-        ev = r.poisson(I.a_lambda, I.a_limit);
-    }
-    double noise = 0.0;  // a_std * z, z drawn once per noise interval
-    if (I.a_std > 0.0) {
-        if (S.fresh_a) {
-            const std::uint64_t nseed = I.seed ^ kSaltAstroNoise;
-            noise = I.a_std * normal_clamped_at(nseed, I.a_indep ? S.noise_a * kStreamStride + a
-                                                                 : S.noise_a);
-            I.noise_a[a] = noise;
-        } else {
-            noise = I.noise_a[a];
+    const std::int64_t first = S[0].step;
+    const int cnt = kSpan ? span_count(I, first, sp.cnt) : (first < I.end_step ? 1 : 0);
+    constexpr bool kEarlyDraws = kSpan && !kWide;
+    // The draws of the launch, as in neuron_role.
+    unsigned long long events = 0;
+    int fresh_at = cnt;
+    double n_fresh = 0.0;
+    if (kEarlyDraws && active) {
+        if (I.a_rate > 0.0)
+            for (int j = 0; j < cnt; ++j) {
+                Draws r(I.seed ^ kSaltAstroPoisson,
+                        static_cast<std::uint64_t>(first + j) * kStreamStride + a);
+                const int ev = r.poisson(I.a_lambda, I.a_limit);
+                events |= static_cast<unsigned long long>(min(ev, 255)) << (8 * j);
+            }
+        if (I.a_std > 0.0) {
+            for (fresh_at = 0; fresh_at < cnt && !S[fresh_at].fresh_a;) ++fresh_at;
+            if (fresh_at < cnt) n_fresh = I.a_std * astro_noise_draw(I, S[fresh_at], a);
         }
     }
-    double ip3_in = 0.0;
-    if (n) {
-        const ShortList l = load_list(I.ring_as, ts);
-        I.ring_as.cnt[ts] = 0;
-        const double v = sum_arrivals<false>(I.ring_as, slot, a, n, l);
-        if (v != 0.0) ip3_in += v;
-    }
-    if (ev > 0) ip3_in += I.a_weight * static_cast<double>(ev);
-    // AstrocytePopulation::update (astrocyte.cpp:307-329)
-    // (the precision study's FP32 form is a separate instantiation: the FP64
-    // kernels carry none of its code)
-    if constexpr (kF32)
-        astro_update_f32(I, ca_tot, ip3_0, tau, delta, ip3_in, noise, ca, ip3, hh);
-    else
-        astro_rk4<false, false>(I.ak, ca_tot, ip3_0, tau, inv_tau, delta, ip3_in, noise, ca, ip3, hh);
-    I.Ca[a] = ca;
-    I.IP3[a] = ip3;
-    I.h[a] = hh;
-    // SIC factor of this step (astrocyte.cpp:331-339), read by the SIC sums
-    // of the arrival step.
-    if (S.fac_now) {
-        const double y = (ca - I.SIC_th) * 1000.0;
-        const double f = y <= 1.0 ? 0.0 : I.SIC_scale * log(y);
-        I.fac[static_cast<std::size_t>(slot) * I.NA + a] = f;
-        if (f != 0.0) I.fac_any[S.fany_now] = 1u;  // every writer stores the same 1
-    }
-    if (I.rec_astro_max > 0 && a < I.rec_astro_max && S.rec_now) {
-        const std::size_t row = S.rec_row;
-        I.rec_Ca[row * I.rec_astro_max + a] = ca;
-        I.rec_IP3[row * I.rec_astro_max + a] = ip3;
+    if (kPdl) grid_dep_wait();
+    // The emission flags fany_ahead steps on start clear (nothing reads or
+    // writes those entries during this launch: see InstDev::fac_any).
+    if (wk.first == 0 && static_cast<int>(threadIdx.x) < cnt && !I.sic_side)
+        I.fac_any[S[threadIdx.x].fany_next] = 0u;
+    if (!active || cnt <= 0) return;
+    std::size_t ts = static_cast<std::size_t>(S[0].slot) * I.ring_as.n_targets + a;
+    std::uint32_t n = __ldcg(I.ring_as.cnt + ts);
+    double ca = I.Ca[a], ip3 = I.IP3[a], hh = I.h[a];
+    double noise = 0.0;  // a_std * z, z drawn once per noise interval
+    if (I.a_std > 0.0 && !S[0].fresh_a) noise = I.noise_a[a];
+    const int n_steps = kSpan ? cnt : 1;
+    for (int j = 0; j < n_steps; ++j) {
+        const StepInfo& T = S[j];
+        const std::int64_t step = first + j;
+        // drive_astrocytes (network.cpp:340-355) and the noise draw
+        // (astrocyte.cpp:307-329)
+        int ev = kEarlyDraws ? static_cast<int>((events >> (8 * j)) & 0xFFu) : 255;
+        if (ev == 255) {
+            ev = 0;
+            if (I.a_rate > 0.0) {
+                Draws r(I.seed ^ kSaltAstroPoisson,
+                        static_cast<std::uint64_t>(step) * kStreamStride + a);
+                ev = r.poisson(I.a_lambda, I.a_limit);
+            }
+        }
+        if (I.a_std > 0.0 && T.fresh_a) {
+            noise = kEarlyDraws && j == fresh_at ? n_fresh : I.a_std * astro_noise_draw(I, T, a);
+            I.noise_a[a] = noise;
+        }
+        double ip3_in = 0.0;
+        if (n) {
+            const ShortList l = load_list(I.ring_as, ts);
+            I.ring_as.cnt[ts] = 0;
+            const double v = sum_arrivals<false>(I.ring_as, T.slot, a, n, l);
+            if (v != 0.0) ip3_in += v;
+        }
+        if (kSpan && j + 1 < cnt) {  // the next step's arrivals, while this one runs
+            ts = static_cast<std::size_t>(S[j + 1].slot) * I.ring_as.n_targets + a;
+            n = __ldcg(I.ring_as.cnt + ts);
+        }
+        if (ev > 0) ip3_in += I.a_weight * static_cast<double>(ev);
+        // AstrocytePopulation::update (astrocyte.cpp:307-329)
+        // (the precision study's FP32 form is a separate instantiation: the FP64
+        // kernels carry none of its code)
+        if constexpr (kF32)
+            astro_update_f32(I, ca_tot, ip3_0, tau, delta, ip3_in, noise, ca, ip3, hh);
+        else
+            astro_rk4<kSpan, kSpan>(I.ak, ca_tot, ip3_0, tau, inv_tau, delta, ip3_in, noise, ca,
+                                    ip3, hh);
+        if (j + 1 == n_steps) {
+            I.Ca[a] = ca;
+            I.IP3[a] = ip3;
+            I.h[a] = hh;
+        }
+        // SIC factor of this step (astrocyte.cpp:331-339), read by the SIC sums
+        // of the arrival step.
+        if (T.fac_now) {
+            const double y = (ca - I.SIC_th) * 1000.0;
+            const double f = y <= 1.0 ? 0.0 : I.SIC_scale * log(y);
+            I.fac[static_cast<std::size_t>(T.eslot) * I.NA + a] = f;
+            // every writer stores the same 1
+            if (f != 0.0 && !I.sic_side) I.fac_any[T.fany_now] = 1u;
+        }
+        if (I.rec_astro_max > 0 && a < I.rec_astro_max && T.rec_now) {
+            const std::size_t row = T.rec_row;
+            I.rec_Ca[row * I.rec_astro_max + a] = ca;
+            I.rec_IP3[row * I.rec_astro_max + a] = ip3;
+        }
     }
 }
 
@@ -1168,71 +1424,72 @@ __device__ void sic_role(const InstDev& I, const StepInfo& S, const Work& wk) {
     if ((threadIdx.x & 31) == 0 && edges) atomicAdd(I.counters + 1, edges);
 }
 
-template <bool kPdl, bool kF32, bool kWide>
-__device__ __forceinline__ int run_role(const InstDev& I, const StepInfo& S, const Work& wk,
-                                        int burst) {
+template <bool kPdl, bool kF32, bool kWide, bool kSpan>
+__device__ __forceinline__ int run_role(const InstDev& I, const StepInfo* S, const Span& sp,
+                                        const Work& wk, int burst) {
     if (wk.role == kRolePush) {
-        push_role<kPdl, kWide>(I, S, wk);
+        push_role<kPdl, kWide, kSpan>(I, S[0], sp, wk);
         return burst;
     }
     if (wk.role == kRoleNeuron) {
-        neuron_role<kPdl, kWide>(I, S, wk);
+        neuron_role<kPdl, kWide, kSpan>(I, S, sp, wk);
     } else if (wk.role == kRoleAstro) {
-        astro_role<kPdl, kF32>(I, S, wk);
-    } else {
-        sic_role<kPdl>(I, S, wk);
+        astro_role<kPdl, kF32, kWide, kSpan>(I, S, sp, wk);
+    } else if (!kSpan) {
+        sic_role<kPdl>(I, S[0], wk);
     }
-    return help_push<kWide>(I, S, wk, burst);
+    return help_push<kWide, kSpan>(I, S[0], sp, wk, burst);
 }
 
-// One step of every resident instance (the body of both kernel forms below).
-// kLoop: block b runs work items b, b + gridDim.x, ... -- several when the
-// grid is one wave of resident blocks (a large step), which saves the
-// per-block staging and scheduling of the items after the first.  Without
-// kLoop the grid covers the work table and block b runs item b alone (a step
-// of a few waves: no loop structure on its path).  No item waits on another
-// within a launch, so any assignment of items to blocks is valid.
-template <bool kF32, bool kLoop>
+// The steps of one launch of every resident instance (the body of the kernel
+// forms below).  kWide: block b runs work items b, b + gridDim.x, ... --
+// several when the grid is one wave of resident blocks (a large step), which
+// saves the per-block staging and scheduling of the items after the first.
+// Otherwise the grid covers the work table and block b runs item b alone (a
+// step of a few waves: no loop structure on its path).  No item waits on
+// another within a launch, so any assignment of items to blocks is valid.
+template <bool kF32, bool kWide, bool kSpan>
 __device__ __forceinline__ void step_body(const InstDev* __restrict__ insts,
-                                          const Work* __restrict__ work, int k, int n_work) {
+                                          const Work* __restrict__ work, const Span& sp,
+                                          int n_work) {
     // Stage the item's instance descriptor and step arithmetic in shared
     // memory (again only when the instance changes).  Both depend only on
     // data written before the chunk started, so this overlaps the tail of
-    // the previous step's grid.
+    // the previous launch's grid.
     __shared__ __align__(16) unsigned char s_raw[sizeof(InstDev)];
-    __shared__ StepInfo s_info;
+    __shared__ StepInfo s_info[kSpan ? kMaxSpan + 1 : 1];
     const InstDev& I = *reinterpret_cast<const InstDev*>(s_raw);
-    if constexpr (!kLoop) {
-        const Work wk = load_work(work + blockIdx.x);  // gridDim.x == n_work
-        const auto* src = reinterpret_cast<const std::uint32_t*>(insts + wk.inst);
+    const auto stage = [&](std::uint32_t inst) {
+        const auto* src = reinterpret_cast<const std::uint32_t*>(insts + inst);
         auto* dst = reinterpret_cast<std::uint32_t*>(s_raw);
         for (unsigned i = threadIdx.x; i < sizeof(InstDev) / 4; i += blockDim.x)
             dst[i] = __ldcg(src + i);
         __syncthreads();
-        if (threadIdx.x < 32) make_step_info(I, I.step0 + k, s_info);
+        if (kSpan)
+            make_span_info(I, sp, s_info);
+        else if (threadIdx.x < 32)
+            make_step_info(I, I.step0 + sp.k, I.step0 + sp.kprev, s_info[0]);
         __syncthreads();
+    };
+    if constexpr (!kWide) {
+        const Work wk = load_work(work + blockIdx.x);  // gridDim.x == n_work
+        stage(wk.inst);
         asm volatile("griddepcontrol.launch_dependents;");  // see below
-        run_role<true, kF32, false>(I, s_info, wk, -1);
+        run_role<true, kF32, false, kSpan>(I, s_info, sp, wk, -1);
         (void)n_work;
         return;
     }
     std::uint32_t staged = 0xFFFFFFFFu;
-    int burst = -1;  // help_push's answer for this step of the staged instance
+    int burst = -1;  // help_push's answer for this launch of the staged instance
     for (int wi = blockIdx.x; wi < n_work; wi += gridDim.x) {
         // Through L2 (never a cached line of an earlier chunk or engine):
         // the descriptors are rewritten by a host copy before every chunk.
         const Work wk = load_work(work + wi);
         if (wk.inst != staged) {  // block-uniform
             __syncthreads();      // the previous item is done with s_raw / s_info
-            const auto* src = reinterpret_cast<const std::uint32_t*>(insts + wk.inst);
-            auto* dst = reinterpret_cast<std::uint32_t*>(s_raw);
-            for (unsigned i = threadIdx.x; i < sizeof(InstDev) / 4; i += blockDim.x)
-                dst[i] = __ldcg(src + i);
-            __syncthreads();
-            if (threadIdx.x < 32) make_step_info(I, I.step0 + k, s_info);
-            __syncthreads();
+            stage(wk.inst);
             if (staged == 0xFFFFFFFFu) {
-                // Programmatic dependent launch: let the next step's grid be
+                // Programmatic dependent launch: let the next launch's grid be
                 // scheduled now.  Each role waits (griddepcontrol.wait) for
                 // this launch's predecessor to complete before touching
                 // state it writes.
@@ -1241,29 +1498,56 @@ __device__ __forceinline__ void step_body(const InstDev* __restrict__ insts,
             staged = wk.inst;
             burst = -1;
         }
-        burst = run_role<true, kF32, true>(I, s_info, wk, burst);
+        burst = run_role<true, kF32, true, kSpan>(I, s_info, sp, wk, burst);
         __syncthreads();  // the role's shared arrays are free for the next item
     }
 }
 
-// Two forms of the step kernel, same arithmetic: step_kernel allows blocks of
-// up to kMaxBlock threads and 128 registers per thread (4 blocks of 128
-// threads per SM; the fewest dependent round trips, for steps of a few
-// waves); step_kernel_wide is for 128-thread blocks at 6 per SM (80
-// registers, some spilled: more warps to hide latency when a step is many
-// waves of blocks).
+// The forms of the step kernel, same arithmetic.  Launches of one step:
+// step_kernel allows blocks of up to kMaxBlock threads and 128 registers per
+// thread (4 blocks of 128 threads per SM; the fewest dependent round trips,
+// for steps of a few waves); step_kernel_wide is for 128-thread blocks at 6 per
+// SM (80 registers, some spilled: more warps to hide latency when a step is
+// many waves of blocks).
 template <bool kF32>
 __global__ void __launch_bounds__(kMaxBlock) step_kernel(const InstDev* __restrict__ insts,
-                                                         const Work* __restrict__ work, int k,
+                                                         const Work* __restrict__ work,
+                                                         const __grid_constant__ Span sp,
                                                          int n_work) {
-    step_body<kF32, false>(insts, work, k, n_work);
+    step_body<kF32, false, false>(insts, work, sp, n_work);
 }
 
 template <bool kF32>
 __global__ void __launch_bounds__(128, 6) step_kernel_wide(const InstDev* __restrict__ insts,
-                                                           const Work* __restrict__ work, int k,
+                                                           const Work* __restrict__ work,
+                                                           const __grid_constant__ Span sp,
                                                            int n_work) {
-    step_body<kF32, true>(insts, work, k, n_work);
+    step_body<kF32, true, false>(insts, work, sp, n_work);
+}
+
+// Launches of several steps (blocks of 128 threads): span_kernel, one item per
+// block, with the registers to keep the step loop free of spills (3 blocks
+// per SM; at 4 per SM the prefetched arrivals were spilled, which waits for
+// them: use_case 2.46 against 2.33 us per step), and span_kernel_wide, one wave
+// of resident blocks, 4 per SM: the step loop needs fewer warps than the
+// single step to hide its loads, and spills cost more (10^6 neurons, us per
+// step: 8 per SM 129, 6 109, 5 93, 4 89, 3 93; with div_newton in the
+// astrocytes 82).  The astrocyte items in a kernel of their own, 4 to 6 blocks
+// per SM, measured the same (81 to 84).
+template <bool kF32>
+__global__ void __launch_bounds__(128, 3) span_kernel(const InstDev* __restrict__ insts,
+                                                      const Work* __restrict__ work,
+                                                      const __grid_constant__ Span sp,
+                                                      int n_work) {
+    step_body<kF32, false, true>(insts, work, sp, n_work);
+}
+
+template <bool kF32>
+__global__ void __launch_bounds__(128, 4) span_kernel_wide(const InstDev* __restrict__ insts,
+                                                           const Work* __restrict__ work,
+                                                           const __grid_constant__ Span sp,
+                                                           int n_work) {
+    step_body<kF32, true, true>(insts, work, sp, n_work);
 }
 
 // Grid-wide barrier of the persistent chunk kernel (all blocks co-resident
@@ -1347,9 +1631,10 @@ __global__ void __launch_bounds__(kMaxBlock) chunk_kernel(const InstDev* __restr
                 __syncthreads();
                 if (threadIdx.x == 0) s_inst = wk.inst;
             }
-            if (threadIdx.x < 32) make_step_info(I, I.step0 + k, s_info);
+            if (threadIdx.x < 32) make_step_info(I, I.step0 + k, I.step0 + k - 1, s_info);
             __syncthreads();
-            if (s_info.step < I.end_step) run_role<false, kF32, false>(I, s_info, wk, -1);
+            const Span sp{k, 1, k - 1, 0, 3, 3, -1, 0};
+            if (s_info.step < I.end_step) run_role<false, kF32, false, false>(I, &s_info, sp, wk, -1);
         }
         if (k + 1 < steps && !grid_sync(gb, gridDim.x)) return;
     }
@@ -1384,7 +1669,7 @@ __global__ void __launch_bounds__(kMaxBlock) sic_batch_kernel(const InstDev* __r
             const std::int64_t a = I.step0 + k + I.sic_lead + j;
             const std::int64_t se = a - I.d_a2n;
             due[j] = a >= I.step0 && se >= 0 && se % I.sic_interval == 0;
-            fac[j] = I.fac + static_cast<std::size_t>(due[j] ? se % I.slots : 0) * I.NA;
+            fac[j] = I.fac + static_cast<std::size_t>(due[j] ? se % I.fac_slots : 0) * I.NA;
             acc[j] = 0.0;
         }
         for (std::uint32_t b0 = 0;; b0 += kSicBatch) {
@@ -1481,16 +1766,31 @@ cudaError_t launch_chunk_persistent(const InstDev* insts, const Work* work, int 
     return cudaLaunchKernelEx(&cfg, chunk_kernel<false>, insts, work, n_work, steps, gb);
 }
 
-int step_wide_blocks_per_sm() {
+namespace {
+
+using StepKernel = void (*)(const InstDev*, const Work*, Span, int);
+
+StepKernel step_kernel_for(StepForm form, bool f32) {
+    switch (form) {
+        case StepForm::kLatency: return f32 ? step_kernel<true> : step_kernel<false>;
+        case StepForm::kWide: return f32 ? step_kernel_wide<true> : step_kernel_wide<false>;
+        case StepForm::kSpan: return f32 ? span_kernel<true> : span_kernel<false>;
+        default: return f32 ? span_kernel_wide<true> : span_kernel_wide<false>;
+    }
+}
+
+}  // namespace
+
+int step_blocks_per_sm(StepForm form, bool f32) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, step_kernel_wide<false>, 128, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, step_kernel_for(form, f32), 128, 0) !=
         cudaSuccess)
         return 0;
     return nb;
 }
 
-cudaError_t launch_step(const InstDev* insts, const Work* work, int n_work, int block, int k,
-                        bool pdl, bool wide, int max_grid, bool f32, cudaStream_t stream) {
+cudaError_t launch_step(const InstDev* insts, const Work* work, int n_work, int block, Span sp,
+                        bool pdl, StepForm form, int max_grid, bool f32, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(max_grid > 0 ? std::min(n_work, max_grid) : n_work));
     cfg.blockDim = dim3(static_cast<unsigned>(block));
@@ -1501,11 +1801,7 @@ cudaError_t launch_step(const InstDev* insts, const Work* work, int n_work, int 
     attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (wide && block == 128)
-        return f32 ? cudaLaunchKernelEx(&cfg, step_kernel_wide<true>, insts, work, k, n_work)
-                   : cudaLaunchKernelEx(&cfg, step_kernel_wide<false>, insts, work, k, n_work);
-    return f32 ? cudaLaunchKernelEx(&cfg, step_kernel<true>, insts, work, k, n_work)
-               : cudaLaunchKernelEx(&cfg, step_kernel<false>, insts, work, k, n_work);
+    return cudaLaunchKernelEx(&cfg, step_kernel_for(form, f32), insts, work, sp, n_work);
 }
 
 }  // namespace asg
