@@ -16,7 +16,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "asg_common.hpp"
@@ -97,8 +96,12 @@ __device__ __forceinline__ void advance_cell(const StepArgs& a, const AstroArray
         astro_rk4(a.k, a.u.Ca_tot, a.u.IP3_0, a.u.tau, a.u.inv_tau, a.u.delta, in, noise, ca, ip3,
                   hh);
     } else {
-        astro_rk4(a.k, s.Ca_tot[i], s.IP3_0[i], s.tau[i], s.inv_tau[i], s.delta[i], in, noise, ca,
-                  ip3, hh);
+        // The reciprocal of tau (div_diff_by): held per cell by the engine;
+        // formed here (IEEE division, correctly rounded) for caller-owned
+        // arrays, once for the whole call.
+        const double tau = s.tau[i];
+        const double inv_tau = kInput == kInputArrayZero ? 1.0 / tau : s.inv_tau[i];
+        astro_rk4(a.k, s.Ca_tot[i], s.IP3_0[i], tau, inv_tau, s.delta[i], in, noise, ca, ip3, hh);
     }
 }
 
@@ -926,92 +929,15 @@ extern "C" int asg_astro_autotune(asg_astro* s, const double* consts, double h_s
 // reach us only as device pointers, or a host framework whose memory pool
 // owns all device memory and forbids allocations of its own during a run.
 // asg_astro_update_noalloc serves them: it updates caller-owned device arrays
-// in place and allocates nothing.  Its only scratch -- the correctly rounded
-// reciprocal of each cell's tau_IP3 that the division in the IP3 rate uses --
-// lives in the file-scope array below.  The array is reserved with this
-// file's device code: when the module is loaded, i.e. at context creation
-// under eager module loading, or at the first call that needs the module
-// (the address lookup below) under CUDA's default lazy loading.  From then
-// on every GPU that uses the library holds it until the process exits.
+// in place and allocates nothing.  One launch and no scratch: the kernel forms
+// the reciprocal of each cell's tau_IP3 itself.  (A kernel of its own that
+// left the reciprocals in a static array cost a launch, a pass over 16 bytes
+// per cell and the array's address lookup on the host: 1,000,003 cells 42.3 ->
+// 31.0 us per call, input copy included.)
 
 namespace asg {
 namespace {
-
-constexpr std::uint32_t kNoAllocMaxCells = 1u << 20;  // 8 MiB of FP64 reciprocals
-__device__ __align__(256) double g_noalloc_inv_tau[kNoAllocMaxCells];
-
-constexpr int kNoAllocMaxDevices = 64;
-struct ScratchAddr {
-    unsigned long long ctx_id = 0;  // driver id of the context the address belongs to
-    double* ptr = nullptr;
-};
-ScratchAddr g_noalloc_scratch[kNoAllocMaxDevices];  // per device ordinal
-std::mutex g_noalloc_mu;
-
-// inv_tau[i] = 1 / tau[i] (IEEE division: the correctly rounded reciprocal).
-__global__ void noalloc_reciprocals(std::uint32_t n, const double* __restrict__ tau,
-                                    double* __restrict__ inv_tau) {
-    const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) inv_tau[i] = 1.0 / tau[i];
-}
-
-// Unique id of the context current on this thread (0 when none is current),
-// from the driver's cuCtxGetCurrent and cuCtxGetId, reached through the
-// runtime's entry-point query so the library need not link libcuda.  Ids are
-// never reused within a process, unlike context handles.
-int current_context_id(unsigned long long* id) {
-    using GetCurrent = int (*)(void**);
-    using GetId = int (*)(void*, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    if (get_current == nullptr || get_id == nullptr) {
-        void* f1 = nullptr;
-        void* f2 = nullptr;
-        cudaDriverEntryPointQueryResult q1{}, q2{};
-        ASG_CUDA(cudaGetDriverEntryPoint("cuCtxGetCurrent", &f1, cudaEnableDefault, &q1));
-        ASG_CUDA(cudaGetDriverEntryPoint("cuCtxGetId", &f2, cudaEnableDefault, &q2));
-        if (q1 != cudaDriverEntryPointSuccess || q2 != cudaDriverEntryPointSuccess || !f1 || !f2)
-            return fail(ASG_ERR_UNSUPPORTED, "driver lacks cuCtxGetCurrent/cuCtxGetId");
-        get_current = reinterpret_cast<GetCurrent>(f1);
-        get_id = reinterpret_cast<GetId>(f2);
-    }
-    void* ctx = nullptr;
-    *id = 0;
-    if (get_current(&ctx) != 0) return fail(ASG_ERR_CUDA, "cuCtxGetCurrent failed");
-    if (ctx != nullptr && get_id(ctx, id) != 0) return fail(ASG_ERR_CUDA, "cuCtxGetId failed");
-    return ASG_OK;
-}
-
-// Device address of the scratch array in the current device's context.  In
-// host code the array's name is only a host-side stand-in, so the address is
-// looked up with cudaGetSymbolAddress, with the device current, once per
-// device -- and again whenever the device's context is a new one (after
-// cudaDeviceReset, or after a host framework released and re-created the
-// primary context), because the cached address belongs to the old context.
-int noalloc_scratch(int dev, double** out) {
-    if (dev < 0 || dev >= kNoAllocMaxDevices)
-        return fail(ASG_ERR_UNSUPPORTED, "device ordinal %d beyond %d", dev, kNoAllocMaxDevices);
-    std::lock_guard<std::mutex> g(g_noalloc_mu);
-    ScratchAddr& e = g_noalloc_scratch[dev];
-    unsigned long long ctx = 0;
-    ASG_TRY(current_context_id(&ctx));
-    if (e.ptr == nullptr || ctx == 0 || ctx != e.ctx_id) {
-        void* p = nullptr;
-        const cudaError_t ce = cudaGetSymbolAddress(&p, g_noalloc_inv_tau);
-        if (ce == cudaErrorMemoryAllocation)
-            return fail(ASG_ERR_OOM,
-                        "asg_astro_update_noalloc: loading the module that holds the %u-cell "
-                        "(8 MiB) scratch array failed: device memory is exhausted",
-                        kNoAllocMaxCells);
-        ASG_CUDA(ce);
-        ASG_TRY(current_context_id(&ctx));  // the lookup made the context current
-        e.ctx_id = ctx;
-        e.ptr = static_cast<double*>(p);
-    }
-    *out = e.ptr;
-    return ASG_OK;
-}
-
+constexpr std::uint32_t kNoAllocMaxCells = 1u << 20;  // the entry point's limit
 }  // namespace
 }  // namespace asg
 
@@ -1052,15 +978,7 @@ extern "C" int asg_astro_update_noalloc(uint32_t n, double* Ca, double* IP3, dou
                          "asg_astro_update_noalloc: a CUDA error from earlier work is pending "
                          "on this thread (%s: %s); nothing was launched",
                          cudaGetErrorName(pending), cudaGetErrorString(pending));
-    int dev = 0;
-    ASG_CUDA(cudaGetDevice(&dev));
-    double* inv_tau = nullptr;
-    ASG_TRY(asg::noalloc_scratch(dev, &inv_tau));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // Every entry this call reads is written first, in stream order, so the
-    // previous call's contents never leak in.
-    asg::noalloc_reciprocals<<<(n + 255) / 256, 256, 0, st>>>(n, tau_IP3, inv_tau);
-    ASG_CUDA(cudaGetLastError());
     asg::StepArgs a;
     std::memset(&a, 0, sizeof a);
     a.n = n;
@@ -1070,11 +988,11 @@ extern "C" int asg_astro_update_noalloc(uint32_t n, double* Ca, double* IP3, dou
     a.shared_noise = shared_noise;
     a.noise_seed = noise_seed;
     a.noise_index = noise_index;
-    const asg::AstroArrays arr{Ca, IP3, h, ip3_input, Ca_tot, IP3_0, tau_IP3, inv_tau, delta_IP3};
-    // Shape 1: one cell per thread with 8-byte accesses, so caller arrays need
-    // no more than double alignment.
+    const asg::AstroArrays arr{Ca, IP3, h, ip3_input, Ca_tot, IP3_0, tau_IP3, nullptr, delta_IP3};
+    // One cell per thread with 8-byte accesses, so caller arrays need no more
+    // than double alignment.
     ASG_CUDA(a.independent
-                 ? (asg::launch_astro<false, asg::kInputArrayZero, true>(1, a, arr, st))
-                 : (asg::launch_astro<false, asg::kInputArrayZero, false>(1, a, arr, st)));
+                 ? (asg::launch_astro<false, asg::kInputArrayZero, true>(4, a, arr, st))
+                 : (asg::launch_astro<false, asg::kInputArrayZero, false>(4, a, arr, st)));
     return ASG_OK;
 }
