@@ -146,13 +146,15 @@ __host__ __device__ __noinline__ inline double ieee_div(double a, double b) { re
 // without a test (div_by's exponent test, as an integer flag).
 __host__ __device__ __forceinline__ unsigned div_out_of_range(double a) {
 #ifdef __CUDA_ARCH__
-    const unsigned biased = (static_cast<unsigned>(__double2hiint(a)) >> 20) & 0x7FFu;
+    const unsigned hi = static_cast<unsigned>(__double2hiint(a));
 #else
     std::uint64_t u;
     __builtin_memcpy(&u, &a, sizeof u);
-    const unsigned biased = static_cast<unsigned>(u >> 52) & 0x7FFu;
+    const unsigned hi = static_cast<unsigned>(u >> 32);
 #endif
-    return (biased - 64u > 1936u) ? 1u : 0u;
+    // biased exponent outside [64, 2000], the sign shifted out: one shift-add
+    // and one comparison
+    return (hi << 1) - (64u << 21) >= (1937u << 21) ? 1u : 0u;
 }
 
 // div_by without its exponent test, for callers that test the numerator

@@ -603,22 +603,21 @@ __device__ __forceinline__ double noise_draw(const InstDev& I, const NeuronK& P,
 // one batch, the counters cleared for the slot's next use, the excitatory
 // sum then the inhibitory one routed as add_synaptic_input does.
 __device__ __forceinline__ void apply_arrivals(const InstDev& I, std::uint32_t slot,
-                                               std::uint32_t c, std::size_t ts_ex,
-                                               std::size_t ts_in, std::uint32_t n_ex,
+                                               std::uint32_t c, std::size_t ts, std::uint32_t n_ex,
                                                std::uint32_t n_in, double v0_ex, double& exc_in,
                                                double& inh_in) {
     ShortList lex{}, lin{};
-    if (n_ex > 1) lex = load_list(I.ring_ex, ts_ex);
-    if (n_in) lin = load_list(I.ring_in, ts_in);
+    if (n_ex > 1) lex = load_list(I.ring_ex, ts);
+    if (n_in) lin = load_list(I.ring_in, ts);
     if (n_ex) {
-        I.ring_ex.cnt[ts_ex] = 0;
+        I.ring_ex.cnt[ts] = 0;
         // one arrival: 0.0 + v, the sum sum_arrivals forms for n = 1
         const double ex =
             n_ex == 1 ? 0.0 + v0_ex : sum_arrivals<false>(I.ring_ex, slot, c, n_ex, lex);
         if (ex != 0.0) add_syn(ex, exc_in, inh_in);
     }
     if (n_in) {
-        I.ring_in.cnt[ts_in] = 0;
+        I.ring_in.cnt[ts] = 0;
         const double in = sum_arrivals<true>(I.ring_in, slot, c, n_in, lin);
         if (in != 0.0) add_syn(-in, exc_in, inh_in);
     }
@@ -629,11 +628,10 @@ struct SynIn {
 };
 
 __device__ __noinline__ SynIn arrivals_out_of_line(const InstDev& I, std::uint32_t slot,
-                                                   std::uint32_t c, std::size_t ts_ex,
-                                                   std::size_t ts_in, std::uint32_t n_ex,
+                                                   std::uint32_t c, std::size_t ts, std::uint32_t n_ex,
                                                    std::uint32_t n_in, double v0_ex) {
     SynIn r{0.0, 0.0};
-    apply_arrivals(I, slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex, r.exc, r.inh);
+    apply_arrivals(I, slot, c, ts, n_ex, n_in, v0_ex, r.exc, r.inh);
     return r;
 }
 
@@ -729,14 +727,14 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
     if (active) {
         // Every input of the first step in one batch of independent loads; a
         // later step's arrivals are loaded while the step before it runs.
-        std::size_t ts_ex = static_cast<std::size_t>(S[0].slot) * I.ring_ex.n_targets + c;
-        std::size_t ts_in = static_cast<std::size_t>(S[0].slot) * I.ring_in.n_targets + c;
-        std::uint32_t n_ex = __ldcg(I.ring_ex.cnt + ts_ex);
-        std::uint32_t n_in = __ldcg(I.ring_in.cnt + ts_in);
+        // (both rings have a target per neuron)
+        std::size_t ts = static_cast<std::size_t>(S[0].slot) * I.N + c;
+        std::uint32_t n_ex = __ldcg(I.ring_ex.cnt + ts);
+        std::uint32_t n_in = __ldcg(I.ring_in.cnt + ts);
         // The first excitatory list value, loaded before the count is known:
         // with a single arrival (the common case) the sum needs no second
         // round trip.
-        double v0_ex = __ldcg(I.ring_ex.lval + ts_ex * kListCap);
+        double v0_ex = __ldcg(I.ring_ex.lval + ts * kListCap);
         // The SIC arriving at the first step; inline, also each later one,
         // formed during the step before it.
         const bool sic_load = S[0].sic_now && !I.fused_sic;
@@ -811,16 +809,16 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
                 // step; the rest go out of line, so the list registers are not
                 // live on the common path.
                 if (n_ex > 1 || n_in != 0u) {
-                    const SynIn a = arrivals_out_of_line(I, T.slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex);
+                    const SynIn a = arrivals_out_of_line(I, T.slot, c, ts, n_ex, n_in, v0_ex);
                     exc_in = a.exc;
                     inh_in = a.inh;
                 } else if (n_ex) {
-                    I.ring_ex.cnt[ts_ex] = 0;
+                    I.ring_ex.cnt[ts] = 0;
                     const double ex = 0.0 + v0_ex;
                     if (ex != 0.0) add_syn(ex, exc_in, inh_in);
                 }
             } else {
-                apply_arrivals(I, T.slot, c, ts_ex, ts_in, n_ex, n_in, v0_ex, exc_in, inh_in);
+                apply_arrivals(I, T.slot, c, ts, n_ex, n_in, v0_ex, exc_in, inh_in);
             }
             if (T.sic_now) {
                 Isic = I.fused_sic ? own_sic(j) : sic_next;
@@ -828,11 +826,10 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
                 if (!kSpan) I.Isic[c] = Isic;
             }
             if (kSpan && j + 1 < cnt) {
-                ts_ex = static_cast<std::size_t>(S[j + 1].slot) * I.ring_ex.n_targets + c;
-                ts_in = static_cast<std::size_t>(S[j + 1].slot) * I.ring_in.n_targets + c;
-                n_ex = __ldcg(I.ring_ex.cnt + ts_ex);
-                n_in = __ldcg(I.ring_in.cnt + ts_in);
-                v0_ex = __ldcg(I.ring_ex.lval + ts_ex * kListCap);
+                ts = static_cast<std::size_t>(S[j + 1].slot) * I.N + c;
+                n_ex = __ldcg(I.ring_ex.cnt + ts);
+                n_in = __ldcg(I.ring_in.cnt + ts);
+                v0_ex = __ldcg(I.ring_ex.lval + ts * kListCap);
                 if (I.sic_side && S[j + 1].sic_now)
                     sic_next = __ldcg(I.sic_val + static_cast<std::size_t>((step + 1) & (I.sic_ring - 1)) * I.N + c);
             }
