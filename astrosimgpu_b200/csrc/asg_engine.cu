@@ -75,21 +75,35 @@ AstroK make_astro_k(const asg_astro_params& a, double h, int substeps) {
     return k;
 }
 
-// Device memory from the stream-ordered allocator: freeing it does not wait
-// for the device (cudaFree would, and stall the chunks in flight).
-struct AsyncBuf {
-    void* p = nullptr;
-    cudaStream_t s = nullptr;
-    cudaError_t alloc(std::size_t bytes, cudaStream_t st) {
-        s = st;
-        return cudaMallocAsync(&p, std::max<std::size_t>(bytes, 16), st);
+// A failed allocation reports ASG_ERR_OOM (a server then waits for memory to
+// free up).
+int need(AsyncBuf& buf, std::size_t bytes, const Scratch& sc) {
+    const cudaError_t e = buf.alloc(bytes, sc);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return fail(ASG_ERR_OOM, "admission: %zu device bytes unavailable", bytes);
     }
-    template <class T>
-    T* as() const { return static_cast<T*>(p); }
-    ~AsyncBuf() {
-        if (p) cudaFreeAsync(p, s);
-    }
+    return e == cudaSuccess ? ASG_OK : cuda_fail(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
+}
+
+// One set's targets on the device (sets of kDeviceEdges edges and more: below
+// it the host checks a set and builds its SIC lists within the ~0.4 ms that
+// the device path's launches and synchronisations take).
+constexpr std::uint32_t kDeviceEdges = 1u << 16;
+
+struct SetTargets {
+    AsyncBuf tg;             // [m], empty for a smaller set
+    std::uint32_t bad = ~0u; // first edge whose target is out of range
 };
+
+__global__ void target_check_kernel(const std::uint32_t* __restrict__ tg, std::uint32_t m,
+                                    std::uint32_t n_targets, std::uint32_t* __restrict__ bad) {
+    std::uint32_t first = 0xFFFFFFFFu;
+    for (std::uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m;
+         e += gridDim.x * blockDim.x)
+        if (tg[e] >= n_targets) first = min(first, e);
+    if (first != 0xFFFFFFFFu) atomicMin(bad, first);
+}
 
 // Transposed in-edge structure of one set, built on the device.  A target's
 // in-edges are numbered p = 0.. in (source, row position) order; bit p of the
@@ -149,35 +163,32 @@ __global__ void ring_pack_kernel(const std::uint32_t* __restrict__ st,
 // then a stable radix sort of (target, edge) pairs and the packing.  Returns
 // with r.words known (the stream synchronised once for it).
 int build_in_ring(std::uint32_t n_src, const std::uint32_t* rs, const std::uint32_t* tg,
-                  std::uint32_t n_targets, cudaStream_t st, InRingDev& r) {
+                  std::uint32_t n_targets, SetTargets& on_device, const Scratch& sc,
+                  InRingDev& r) {
     NvtxRange nvtx("admission: in-edge numbering (arrival rings)");
     const std::uint32_t m = rs[n_src];
     const std::uint32_t n = n_targets;
+    const cudaStream_t st = sc.stream;
     r.m = m;
     if (m >= (1u << 31)) return fail(ASG_ERR_UNSUPPORTED, "a set of %u edges (at most 2^31-1)", m);
-    // Scratch beyond the arena: a failed allocation reports ASG_ERR_OOM (a
-    // server then waits for memory to free up).
-    auto need = [&](AsyncBuf& buf, std::size_t bytes) -> int {
-        const cudaError_t e = buf.alloc(bytes, st);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            return fail(ASG_ERR_OOM, "in-edge numbering: %zu device bytes unavailable", bytes);
-        }
-        return e == cudaSuccess ? ASG_OK : cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
-    };
-    ASG_TRY(need(r.wbase, (static_cast<std::size_t>(n) + 1) * 4));
-    ASG_TRY(need(r.edge, static_cast<std::size_t>(m) * 8));
+    ASG_TRY(need(r.wbase, (static_cast<std::size_t>(n) + 1) * 4, sc));
+    ASG_TRY(need(r.edge, static_cast<std::size_t>(m) * 8, sc));
     if (m == 0) {
         ASG_CUDA(cudaMemsetAsync(r.wbase.p, 0, (static_cast<std::size_t>(n) + 1) * 4, st));
         r.words = 0;
         return ASG_OK;
     }
     AsyncBuf keys, keys_out, vals, vals_out, deg, seg, words, tmp;
-    for (AsyncBuf* buf : {&keys, &keys_out, &vals, &vals_out})
-        ASG_TRY(need(*buf, static_cast<std::size_t>(m) * 4));
+    std::swap(keys.p, on_device.tg.p);
+    keys.from = sc;
+    if (keys.p == nullptr) {
+        ASG_TRY(need(keys, static_cast<std::size_t>(m) * 4, sc));
+        ASG_CUDA(cudaMemcpyAsync(keys.p, tg, static_cast<std::size_t>(m) * 4, cudaMemcpyDefault, st));
+    }
+    for (AsyncBuf* buf : {&keys_out, &vals, &vals_out})
+        ASG_TRY(need(*buf, static_cast<std::size_t>(m) * 4, sc));
     for (AsyncBuf* buf : {&deg, &seg, &words})
-        ASG_TRY(need(*buf, (static_cast<std::size_t>(n) + 1) * 4));
-    ASG_CUDA(cudaMemcpyAsync(keys.p, tg, static_cast<std::size_t>(m) * 4, cudaMemcpyDefault, st));
+        ASG_TRY(need(*buf, (static_cast<std::size_t>(n) + 1) * 4, sc));
     ASG_CUDA(cudaMemsetAsync(deg.p, 0, (static_cast<std::size_t>(n) + 1) * 4, st));
     const unsigned blocks = 4096;
     ring_count_kernel<<<blocks, 256, 0, st>>>(keys.as<std::uint32_t>(), m, deg.as<std::uint32_t>());
@@ -194,7 +205,7 @@ int build_in_ring(std::uint32_t n_src, const std::uint32_t* rs, const std::uint3
                                              vals_out.as<std::uint32_t>(), static_cast<int>(m), 0,
                                              end_bit, st));
     std::size_t b = std::max(b_scan, b_sort);
-    ASG_TRY(need(tmp, b));
+    ASG_TRY(need(tmp, b, sc));
     ASG_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, b, deg.as<std::uint32_t>(),
                                            seg.as<std::uint32_t>(), static_cast<int>(n) + 1, st));
     b = std::max(b_scan, b_sort);
@@ -293,6 +304,141 @@ SicHost make_sic(std::uint32_t NA, const std::uint32_t* rs, const std::uint32_t*
     return s;
 }
 
+// The same lists built on the device for an uncut chain (one part): in-degrees
+// (their maximum decides the SIC form), a stable sort of (target, astrocyte)
+// pairs, and one thread per target that walks its run of the sorted pairs
+// twice -- to count its entries, a slice being as long as its longest list,
+// and to write them.  (The host's list of lists took 4 of the 15 ms that
+// admitting a 40,000-neuron network took.)
+struct SicDev {
+    AsyncBuf deg;        // [N + 1]
+    AsyncBuf soff, ent;  // [npad / 32 + 1], [ent_n]
+    std::uint32_t ent_n = 0, max_edges = 0;
+};
+
+__global__ void sic_source_kernel(const std::uint32_t* __restrict__ rs, std::uint32_t NA,
+                                  std::uint32_t* __restrict__ src) {
+    for (std::uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < NA;
+         a += gridDim.x * blockDim.x)
+        for (std::uint32_t e = rs[a]; e < rs[a + 1]; ++e) src[e] = a;
+}
+
+// Calls put(astrocyte << 8 | multiplicity) for target t's entries in order.
+template <class Put>
+__device__ __forceinline__ void sic_entries(const std::uint32_t* __restrict__ astro,
+                                            std::uint32_t begin, std::uint32_t end, Put put) {
+    for (std::uint32_t i = begin; i < end;) {
+        const std::uint32_t a = astro[i];
+        std::uint32_t m = 1;
+        while (m < 255u && i + m < end && astro[i + m] == a) ++m;
+        put((a << 8) | m);
+        i += m;
+    }
+}
+
+// One warp per slice of 32 targets.
+__global__ void sic_slice_kernel(const std::uint32_t* __restrict__ seg,
+                                 const std::uint32_t* __restrict__ astro, std::uint32_t N,
+                                 std::uint32_t npad, std::uint32_t* __restrict__ slice_len) {
+    const std::uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= npad) return;  // npad is a multiple of 32: whole warps
+    std::uint32_t n = 0;
+    if (t < N) sic_entries(astro, seg[t], seg[t + 1], [&](std::uint32_t) { ++n; });
+    for (int o = 16; o > 0; o >>= 1) n = max(n, __shfl_xor_sync(0xFFFFFFFFu, n, o));
+    if ((t & 31u) == 0) slice_len[t >> 5] = n * 32u;
+    if (t == 0) slice_len[npad >> 5] = 0u;  // the scan's last entry is the total
+}
+
+__global__ void sic_fill_kernel(const std::uint32_t* __restrict__ seg,
+                                const std::uint32_t* __restrict__ astro, std::uint32_t N,
+                                const std::uint32_t* __restrict__ soff,
+                                std::uint32_t* __restrict__ ent) {
+    const std::uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= N) return;
+    std::uint32_t o = soff[t >> 5] + (t & 31u);
+    sic_entries(astro, seg[t], seg[t + 1], [&](std::uint32_t e) {
+        ent[o] = e;
+        o += 32u;
+    });
+}
+
+// In-degrees of the SIC set and their maximum (one synchronisation).
+int sic_degrees(const SetTargets& t, std::uint32_t m, std::uint32_t N, const Scratch& sc, SicDev& r) {
+    AsyncBuf mx, tmp;
+    ASG_TRY(need(r.deg, (static_cast<std::size_t>(N) + 1) * 4, sc));
+    ASG_TRY(need(mx, 4, sc));
+    ASG_CUDA(cudaMemsetAsync(r.deg.p, 0, (static_cast<std::size_t>(N) + 1) * 4, sc.stream));
+    ring_count_kernel<<<4096, 256, 0, sc.stream>>>(t.tg.as<std::uint32_t>(), m,
+                                                   r.deg.as<std::uint32_t>());
+    ASG_CUDA(cudaGetLastError());
+    std::size_t b = 0;
+    ASG_CUDA(cub::DeviceReduce::Max(nullptr, b, r.deg.as<std::uint32_t>(), mx.as<std::uint32_t>(),
+                                    static_cast<int>(N), sc.stream));
+    ASG_TRY(need(tmp, b, sc));
+    ASG_CUDA(cub::DeviceReduce::Max(tmp.p, b, r.deg.as<std::uint32_t>(), mx.as<std::uint32_t>(),
+                                    static_cast<int>(N), sc.stream));
+    ASG_CUDA(cudaMemcpyAsync(&r.max_edges, mx.p, 4, cudaMemcpyDeviceToHost, sc.stream));
+    ASG_CUDA(cudaStreamSynchronize(sc.stream));
+    return ASG_OK;
+}
+
+int build_sic(const std::uint32_t* rs, std::uint32_t NA, SetTargets& t, std::uint32_t m,
+              std::uint32_t N, std::uint32_t npad, const Scratch& sc, SicDev& r) {
+    NvtxRange nvtx("admission: SIC lists");
+    const std::uint32_t slices = npad / 32;
+    AsyncBuf d_rs, src, tg_out, astro, seg, len, tmp;
+    ASG_TRY(need(d_rs, (static_cast<std::size_t>(NA) + 1) * 4, sc));
+    for (AsyncBuf* buf : {&src, &tg_out, &astro})
+        ASG_TRY(need(*buf, static_cast<std::size_t>(m) * 4, sc));
+    ASG_TRY(need(seg, (static_cast<std::size_t>(N) + 1) * 4, sc));
+    for (AsyncBuf* buf : {&len, &r.soff})
+        ASG_TRY(need(*buf, (static_cast<std::size_t>(slices) + 1) * 4, sc));
+    ASG_CUDA(cudaMemcpyAsync(d_rs.p, rs, (static_cast<std::size_t>(NA) + 1) * 4, cudaMemcpyDefault,
+                             sc.stream));
+    sic_source_kernel<<<4096, 256, 0, sc.stream>>>(d_rs.as<std::uint32_t>(), NA, src.as<std::uint32_t>());
+    ASG_CUDA(cudaGetLastError());
+    int end_bit = 1;
+    while (end_bit < 32 && (1ull << end_bit) < N) ++end_bit;
+    auto* tg = t.tg.as<std::uint32_t>();
+    std::size_t b1 = 0, b2 = 0, b3 = 0;
+    ASG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b1, r.deg.as<std::uint32_t>(),
+                                           seg.as<std::uint32_t>(), static_cast<int>(N) + 1, sc.stream));
+    ASG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b2, len.as<std::uint32_t>(),
+                                           r.soff.as<std::uint32_t>(), static_cast<int>(slices) + 1,
+                                           sc.stream));
+    ASG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b3, tg, tg_out.as<std::uint32_t>(),
+                                             src.as<std::uint32_t>(), astro.as<std::uint32_t>(),
+                                             static_cast<int>(m), 0, end_bit, sc.stream));
+    std::size_t b = std::max({b1, b2, b3});
+    const std::size_t cap = b;
+    ASG_TRY(need(tmp, cap, sc));
+    ASG_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, b, r.deg.as<std::uint32_t>(),
+                                           seg.as<std::uint32_t>(), static_cast<int>(N) + 1, sc.stream));
+    b = cap;
+    ASG_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, b, tg, tg_out.as<std::uint32_t>(),
+                                             src.as<std::uint32_t>(), astro.as<std::uint32_t>(),
+                                             static_cast<int>(m), 0, end_bit, sc.stream));
+    sic_slice_kernel<<<(npad + 127) / 128, 128, 0, sc.stream>>>(
+        seg.as<std::uint32_t>(), astro.as<std::uint32_t>(), N, npad, len.as<std::uint32_t>());
+    ASG_CUDA(cudaGetLastError());
+    b = cap;
+    ASG_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, b, len.as<std::uint32_t>(),
+                                           r.soff.as<std::uint32_t>(), static_cast<int>(slices) + 1,
+                                           sc.stream));
+    std::uint32_t total = 0;
+    ASG_CUDA(cudaMemcpyAsync(&total, r.soff.as<std::uint32_t>() + slices, 4, cudaMemcpyDeviceToHost,
+                             sc.stream));
+    ASG_CUDA(cudaStreamSynchronize(sc.stream));
+    r.ent_n = std::max<std::uint32_t>(total, 1);
+    ASG_TRY(need(r.ent, static_cast<std::size_t>(r.ent_n) * 4, sc));
+    ASG_CUDA(cudaMemsetAsync(r.ent.p, 0, static_cast<std::size_t>(r.ent_n) * 4, sc.stream));
+    sic_fill_kernel<<<(N + 127) / 128, 128, 0, sc.stream>>>(
+        seg.as<std::uint32_t>(), astro.as<std::uint32_t>(), N, r.soff.as<std::uint32_t>(),
+        r.ent.as<std::uint32_t>());
+    ASG_CUDA(cudaGetLastError());
+    return ASG_OK;
+}
+
 // The first index e in [0, m) with bad(e), or m; large ranges are scanned
 // on all of the host's cores.
 template <class Bad>
@@ -305,7 +451,7 @@ std::uint32_t first_bad(std::uint32_t m, Bad bad) {
     return first;
 }
 
-int check_csr(const char* name, const asg_csr& c, std::uint32_t n_src, std::uint32_t n_tgt) {
+int check_csr(const char* name, const asg_csr& c, std::uint32_t n_src) {
     if (c.n_sources != n_src)
         return fail(ASG_ERR_ARG, "%s: n_sources %u, expected %u", name, c.n_sources, n_src);
     if (n_src > 0 && (c.row_start == nullptr))
@@ -315,12 +461,32 @@ int check_csr(const char* name, const asg_csr& c, std::uint32_t n_src, std::uint
     const std::uint32_t s =
         first_bad(n_src, [&](std::uint32_t i) { return c.row_start[i + 1] < c.row_start[i]; });
     if (s < n_src) return fail(ASG_ERR_ARG, "%s: row_start decreases at %u", name, s);
-    const std::uint32_t m = c.row_start[n_src];
-    if (m > 0 && c.target == nullptr) return fail(ASG_ERR_ARG, "%s: target is NULL", name);
-    const std::uint32_t e = first_bad(m, [&](std::uint32_t i) { return c.target[i] >= n_tgt; });
-    if (e < m)
-        return fail(ASG_ERR_ARG, "%s: target[%u] = %u out of range (%u)", name, e, c.target[e],
-                    n_tgt);
+    if (c.row_start[n_src] > 0 && c.target == nullptr)
+        return fail(ASG_ERR_ARG, "%s: target is NULL", name);
+    return ASG_OK;
+}
+
+// Targets in range: a small set on the host, a larger one uploaded (it is
+// needed there next) and scanned on the device; `t.bad` is read once the
+// stream has been synchronised.
+int scan_targets(const asg_csr& c, std::uint32_t n_src, std::uint32_t n_tgt, const Scratch& sc,
+                 AsyncBuf& flag, SetTargets& t) {
+    const std::uint32_t m = n_src ? c.row_start[n_src] : 0;
+    const bool here = m < kDeviceEdges || m >= (1u << 31);
+    if (here || need(flag, 4, sc) != ASG_OK ||
+        need(t.tg, static_cast<std::size_t>(m) * 4, sc) != ASG_OK) {
+        clear_error();  // no room for the scan there
+        const std::uint32_t e = first_bad(m, [&](std::uint32_t i) { return c.target[i] >= n_tgt; });
+        if (e < m) t.bad = e;
+        return ASG_OK;
+    }
+    ASG_CUDA(cudaMemsetAsync(flag.p, 0xFF, 4, sc.stream));
+    ASG_CUDA(cudaMemcpyAsync(t.tg.p, c.target, static_cast<std::size_t>(m) * 4, cudaMemcpyDefault,
+                             sc.stream));
+    target_check_kernel<<<2048, 256, 0, sc.stream>>>(t.tg.as<std::uint32_t>(), m, n_tgt,
+                                                     flag.as<std::uint32_t>());
+    ASG_CUDA(cudaGetLastError());
+    ASG_CUDA(cudaMemcpyAsync(&t.bad, flag.p, 4, cudaMemcpyDeviceToHost, sc.stream));
     return ASG_OK;
 }
 
@@ -328,7 +494,7 @@ int check_uniform(const char* name, const asg_csr& c, std::uint32_t n_src, doubl
                   const asg_stp& stp) {
     if (n_src == 0) return ASG_OK;
     const std::uint32_t m = c.row_start[n_src];
-    const std::uint32_t e = first_bad(m, [&](std::uint32_t i) {
+    const std::uint32_t e = !c.weight && !c.delay_steps ? m : first_bad(m, [&](std::uint32_t i) {
         return (c.weight && c.weight[i] != w) || (c.delay_steps && c.delay_steps[i] != d);
     });
     if (e < m && c.weight && c.weight[e] != w)
@@ -371,11 +537,47 @@ std::size_t align256(std::size_t x) { return (x + 255) & ~static_cast<std::size_
 
 }  // namespace
 
+void Instance::drop_span() {
+    if (span_total) span_total->fetch_sub(span_bytes);
+    span_total = nullptr;
+}
+
 Instance::~Instance() {
+    drop_span();
     for (int p = 0; p < 2; ++p) {
-        if (log_h[p]) cudaFreeHost(log_h[p]);
-        if (rec_h[p]) cudaFreeHost(rec_h[p]);
+        if (log_h[p]) host_pool->give(log_h[p], log_bytes);
+        if (rec_h[p]) host_pool->give(rec_h[p], rec_bytes);
     }
+}
+
+cudaError_t HostPool::take(std::size_t bytes, void** p) {
+    {
+        std::lock_guard<std::mutex> g(mu);
+        for (std::size_t i = 0; i < kept.size(); ++i) {
+            if (kept[i].first != bytes) continue;
+            *p = kept[i].second;
+            held -= bytes;
+            kept.erase(kept.begin() + static_cast<std::ptrdiff_t>(i));
+            return cudaSuccess;
+        }
+    }
+    return cudaHostAlloc(p, bytes, cudaHostAllocMapped);
+}
+
+void HostPool::give(void* p, std::size_t bytes) {
+    {
+        std::lock_guard<std::mutex> g(mu);
+        if (held + bytes <= kKeep) {
+            kept.emplace_back(bytes, p);
+            held += bytes;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+HostPool::~HostPool() {
+    for (auto& k : kept) cudaFreeHost(k.second);
 }
 
 Engine::Engine(const EngineConfig& c) : cfg(c) {}
@@ -400,7 +602,11 @@ Engine::~Engine() {
     }
     insts.clear();
     if (side) cudaStreamDestroy(side);
-    if (upload) cudaStreamDestroy(upload);
+    if (upload) {
+        cudaStreamSynchronize(upload);
+        cudaStreamDestroy(upload);
+    }
+    if (pool) cudaMemPoolDestroy(pool);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -416,14 +622,22 @@ int Engine::init() {
     if (cfg.block <= 0) cfg.block = 128;
     if (cfg.block > 512 || cfg.block % 32 != 0)
         return fail(ASG_ERR_ARG, "block size %d must be a multiple of 32 in [32, 512]", cfg.block);
-    if (cfg.mem_budget == 0) {
-        std::size_t fr = 0, tot = 0;
-        ASG_CUDA(cudaMemGetInfo(&fr, &tot));
+    std::size_t fr = 0, tot = 0;
+    ASG_CUDA(cudaMemGetInfo(&fr, &tot));
+    free_at_init = fr;
+    budget_given = cfg.mem_budget != 0;
+    if (cfg.mem_budget == 0)
         cfg.mem_budget = static_cast<std::uint64_t>(0.9 * static_cast<double>(fr));
-    }
     ASG_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     ASG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     ASG_CUDA(cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking));
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = cfg.device;
+    ASG_CUDA(cudaMemPoolCreate(&pool, &props));
+    std::uint64_t keep = 2ull << 30;  // unused memory held
+    ASG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
     ASG_CUDA(cudaEventCreateWithFlags(&ev_side_fork, cudaEventDisableTiming));
     ASG_CUDA(cudaEventCreateWithFlags(&ev_side_join, cudaEventDisableTiming));
     for (int q = 0; q < kSideEvents; ++q) {
@@ -496,6 +710,17 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
                     std::int64_t end, bool keep_spikes, bool check_budget,
                     std::unique_ptr<Instance>* out) {
     NvtxRange nvtx("admission: prepare instance");
+    const int st = prepare_instance(d, rec, first, end, keep_spikes, check_budget, out);
+    if (!cfg.keep_memory) {  // the scratch goes back (its frees are on the stream)
+        cudaStreamSynchronize(upload);
+        cudaMemPoolTrimTo(pool, 0);
+    }
+    return st;
+}
+
+int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* rec,
+                             std::int64_t first, std::int64_t end, bool keep_spikes,
+                             bool check_budget, std::unique_ptr<Instance>* out) {
     // Touches no state the chunks in flight use: the tables are prepared and
     // uploaded on the upload stream into a new arena, so a serving loop can
     // run this on another thread while the engine's stream keeps stepping.
@@ -510,10 +735,33 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
     if (N > 0 && (d.V_reset == nullptr || d.b == nullptr))
         return fail(ASG_ERR_ARG, "per-cell V_reset and b are required");
     if (first < 0 || end < first) return fail(ASG_ERR_ARG, "bad step range");
-    ASG_TRY(check_csr("exc_primary", d.exc_primary, NE, N));
-    ASG_TRY(check_csr("inh_primary", d.inh_primary, NI, N));
-    ASG_TRY(check_csr("neuron_astro", d.neuron_astro, NE, std::max(NA, 1u)));
-    ASG_TRY(check_csr("astro_neuron", d.astro_neuron, NA, N));
+    ASG_TRY(check_csr("exc_primary", d.exc_primary, NE));
+    ASG_TRY(check_csr("inh_primary", d.inh_primary, NI));
+    ASG_TRY(check_csr("neuron_astro", d.neuron_astro, NE));
+    ASG_TRY(check_csr("astro_neuron", d.astro_neuron, NA));
+    const Scratch sc{upload, pool};
+    SetTargets on_exc, on_inh, on_n2a, on_a2n;
+    {
+        struct {
+            const char* name;
+            const asg_csr* c;
+            std::uint32_t n_src, n_tgt;
+            SetTargets* t;
+        } sets[] = {{"exc_primary", &d.exc_primary, NE, N, &on_exc},
+                    {"inh_primary", &d.inh_primary, NI, N, &on_inh},
+                    {"neuron_astro", &d.neuron_astro, NE, std::max(NA, 1u), &on_n2a},
+                    {"astro_neuron", &d.astro_neuron, NA, N, &on_a2n}};
+        AsyncBuf flags[4];
+        int st = ASG_OK;
+        for (int k = 0; k < 4 && st == ASG_OK; ++k)
+            st = scan_targets(*sets[k].c, sets[k].n_src, sets[k].n_tgt, sc, flags[k], *sets[k].t);
+        ASG_CUDA(cudaStreamSynchronize(upload));  // the flags, also before an early return
+        ASG_TRY(st);
+        for (const auto& k : sets)
+            if (k.t->bad != ~0u)
+                return fail(ASG_ERR_ARG, "%s: target[%u] = %u out of range (%u)", k.name, k.t->bad,
+                            k.c->target[k.t->bad], k.n_tgt);
+    }
     if (NA == 0 && d.neuron_astro.n_sources && d.neuron_astro.row_start &&
         d.neuron_astro.row_start[NE] > 0)
         return fail(ASG_ERR_ARG, "neuron_astro has edges but there are no astrocytes");
@@ -593,8 +841,14 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
     // its neuron thread, which saves the SIC role's blocks (a third of the
     // step's); a smaller network keeps the SIC role, which runs beside the
     // neuron role (lower latency).
+    SicDev sic_dev;
+    const std::uint32_t sic_m = rs_of(d.astro_neuron)[d.astro_neuron.n_sources];
+    if (on_a2n.tg.p != nullptr) ASG_TRY(sic_degrees(on_a2n, sic_m, N, sc, sic_dev));
     const std::uint32_t sic_mx =
-        NA > 0 ? sic_max_edges(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N) : 0;
+        NA == 0 ? 0
+        : on_a2n.tg.p != nullptr
+            ? sic_dev.max_edges
+            : sic_max_edges(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N);
     const bool fuse_auto =
         D.d_a2n < 2 || ((N >= (1u << 16) || cfg.large_total) && sic_mx <= kSicEdgesPerPart);
     D.fused_sic = cfg.sic_mode == 1 ? 1 : cfg.sic_mode == 2 ? (D.d_a2n >= 2 ? 0 : 1)
@@ -662,9 +916,10 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
 
     // Host preprocessing of the tables.
     InRingDev rex, rin, ras;
-    ASG_TRY(build_in_ring(NE, rs_of(d.exc_primary), d.exc_primary.target, N, upload, rex));
-    ASG_TRY(build_in_ring(NI, rs_of(d.inh_primary), d.inh_primary.target, N, upload, rin));
-    ASG_TRY(build_in_ring(NE, rs_of(d.neuron_astro), d.neuron_astro.target, NA, upload, ras));
+    ASG_TRY(build_in_ring(NE, rs_of(d.exc_primary), d.exc_primary.target, N, on_exc, sc, rex));
+    ASG_TRY(build_in_ring(NI, rs_of(d.inh_primary), d.inh_primary.target, N, on_inh, sc, rin));
+    ASG_TRY(build_in_ring(NE, rs_of(d.neuron_astro), d.neuron_astro.target, NA, on_n2a, sc,
+                          ras));
     // SIC parts: about kSicEdgesPerPart edges each, at most d_a2n - 1 (the
     // first part of arrival step A runs at step A - P and reads the factors
     // of step A - d_a2n, written by an earlier launch).
@@ -707,8 +962,17 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
         }
         I.span_max = std::max(1, L);
     }
-    SicHost sic = make_sic(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N,
-                           static_cast<std::uint32_t>(D.sic_parts), D.sic_npad);
+    SicHost sic;
+    bool sic_on_device = on_a2n.tg.p != nullptr && D.sic_parts == 1;
+    if (sic_on_device) {
+        const int st = build_sic(rs_of(d.astro_neuron), NA, on_a2n, sic_m, N, D.sic_npad, sc, sic_dev);
+        if (st != ASG_OK && st != ASG_ERR_OOM) return st;
+        if (st == ASG_ERR_OOM) clear_error();  // no room for the sort: on the host
+        sic_on_device = st == ASG_OK;
+    }
+    if (!sic_on_device)
+        sic = make_sic(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N,
+                       static_cast<std::uint32_t>(D.sic_parts), D.sic_npad);
 
     // Initial state (reference defaults where not given).
     std::vector<double> V0, Ca0, IP30, h0, stp_x(N, 1.0), stp_u(N, d.stp.U), stp_t(N, -1e12);
@@ -790,8 +1054,13 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
     add_seg(D.spk_packed, 3 * kHeaderStride * 8, nullptr);
     add_seg(D.spk_meta, 3 * std::max<std::size_t>(N, 1) * 16, nullptr);
     add_seg(D.spk_val, 3 * std::max<std::size_t>(N, 1) * 16, nullptr);
-    add_seg(D.sic_soff, sic.soff.size() * 4, sic.soff.data());
-    add_seg(D.sic_ent, sic.ent.size() * 4, sic.ent.data());
+    if (sic_on_device) {  // device copies
+        add_seg(D.sic_soff, (static_cast<std::size_t>(D.sic_npad) / 32 + 1) * 4, sic_dev.soff.p);
+        add_seg(D.sic_ent, static_cast<std::size_t>(sic_dev.ent_n) * 4, sic_dev.ent.p);
+    } else {
+        add_seg(D.sic_soff, sic.soff.size() * 4, sic.soff.data());
+        add_seg(D.sic_ent, sic.ent.size() * 4, sic.ent.data());
+    }
     add_seg(D.fac, S * std::max<std::size_t>(a8, 8), nullptr);
     add_seg(D.fac_any, (S + 1) * 4, nullptr);
     add_seg(D.noise_n, n8, nullptr);
@@ -806,7 +1075,10 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
         return fail(ASG_ERR_OOM, "instance needs %zu device bytes; %llu of %llu in use", total,
                     static_cast<unsigned long long>(resident_bytes),
                     static_cast<unsigned long long>(cfg.mem_budget));
-    ASG_TRY(I.arena.alloc(total, false));
+    if (injected_alloc_failure())
+        return fail(ASG_ERR_OOM, "device allocation of %zu bytes refused (injected failure)", total);
+    const Scratch keep{upload, cfg.keep_memory ? pool : nullptr};
+    ASG_TRY(need(I.arena, total, keep));
     I.arena_bytes = total;
     {
         char* base = I.arena.as<char>();
@@ -829,19 +1101,23 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
         ASG_CUDA(cudaStreamSynchronize(upload));  // host sources go out of scope
     }
 
-    // The span buffer comes out of what the budget leaves free; without it
-    // the instance runs one step per launch.
+    // The span buffers stay within a budget the caller gave; beside the default
+    // one they take at most half of what it leaves free.  Without one the
+    // instance runs one step per launch.
     if (I.span_max > 1) {
         const std::size_t cap = static_cast<std::size_t>(N) * I.span_max;
         const std::size_t rec = align256(2 * cap * 16);
         const std::size_t fac = D.sic_side ? 0 : align256(static_cast<std::size_t>(D.d_a2n + kMaxSpan) * a8);
         const std::size_t any = align256((static_cast<std::size_t>(D.d_a2n) + 2 * kMaxSpan) * 4);
         const std::size_t bytes = 2 * rec + fac + any;
-        const std::uint64_t used = resident_bytes + total;
-        const std::uint64_t left = cfg.mem_budget > used ? cfg.mem_budget - used : 0;
-        std::size_t fr = 0, tot = 0;
-        ASG_CUDA(cudaMemGetInfo(&fr, &tot));
-        if (fr >= bytes && fr - bytes >= left && I.span.alloc(bytes, false) == ASG_OK) {
+        const std::uint64_t spans = span_bytes.fetch_add(bytes) + bytes;
+        const std::uint64_t spare =
+            free_at_init > cfg.mem_budget ? (free_at_init - cfg.mem_budget) / 2 : 0;
+        const bool room = budget_given ? resident_bytes + total + spans <= cfg.mem_budget
+                                       : spans <= spare;
+        I.span_bytes = bytes;
+        I.span_total = &span_bytes;
+        if (room && need(I.span, bytes, keep) == ASG_OK) {
             char* p = I.span.as<char>();
             ASG_CUDA(cudaMemsetAsync(p + 2 * rec, 0, fac + any, upload));
             ASG_CUDA(cudaStreamSynchronize(upload));
@@ -852,6 +1128,7 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
             I.span_fany = reinterpret_cast<std::uint32_t*>(p + 2 * rec + fac);
         } else {
             clear_error();
+            I.drop_span();
             I.span_max = 1;
         }
     }
@@ -875,13 +1152,20 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
     I.max_chunk = cfg.chunk_steps;
     const std::size_t rec_doubles =
         static_cast<std::size_t>(I.rec_rows) * (2 * D.rec_astro_max + 2 * D.rec_neuron_max) + 1;
+    // (a server's sizes are rounded up, so that a later request finds them)
+    I.host_pool = host_pool;
+    I.log_bytes = static_cast<std::size_t>(I.log_cap) * 8;
+    I.rec_bytes = rec_doubles * 8;
+    if (cfg.keep_memory) {
+        I.log_bytes = HostPool::rounded(I.log_bytes);
+        I.rec_bytes = HostPool::rounded(I.rec_bytes);
+    }
     for (int p = 0; p < 2; ++p) {
         if (D.rec_spikes) {
-            ASG_CUDA(cudaHostAlloc(&I.log_h[p], static_cast<std::size_t>(I.log_cap) * 8,
-                                   cudaHostAllocMapped));
+            ASG_CUDA(host_pool->take(I.log_bytes, reinterpret_cast<void**>(&I.log_h[p])));
             ASG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&I.log_d[p]), I.log_h[p], 0));
         }
-        ASG_CUDA(cudaHostAlloc(&I.rec_h[p], rec_doubles * 8, cudaHostAllocMapped));
+        ASG_CUDA(host_pool->take(I.rec_bytes, reinterpret_cast<void**>(&I.rec_h[p])));
         ASG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&I.rec_d[p]), I.rec_h[p], 0));
     }
     D.spike_log_cap = D.rec_spikes ? I.log_cap : 0;

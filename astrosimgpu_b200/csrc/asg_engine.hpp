@@ -7,9 +7,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -24,17 +26,75 @@ struct SpikeRec {
     std::uint32_t source;
 };
 
+// Where admission takes device memory: a stream-ordered pool of the engine's
+// own.  (The default pool gives its memory back at every synchronisation and
+// the next allocation maps it again; cudaMalloc and cudaFree wait for the
+// device and, beside running chunks, took from 0.4 to tens of ms each.)  A
+// server's pool also holds the arenas and keeps up to 2 GB between requests;
+// other engines trim it after each admission and take their arenas, which
+// stay, from cudaMalloc (pool = nullptr).
+struct Scratch {
+    cudaStream_t stream;
+    cudaMemPool_t pool;
+};
+
+// Device memory from there.  Freeing pool memory does not wait for the device
+// (cudaFree would, and stall the chunks in flight): its last user must have
+// finished, or be on the same stream.
+struct AsyncBuf {
+    void* p = nullptr;
+    Scratch from{};
+    AsyncBuf() = default;
+    AsyncBuf(const AsyncBuf&) = delete;
+    AsyncBuf& operator=(const AsyncBuf&) = delete;
+    cudaError_t alloc(std::size_t bytes, const Scratch& sc) {
+        from = sc;
+        bytes = std::max<std::size_t>(bytes, 16);
+        return sc.pool ? cudaMallocFromPoolAsync(&p, bytes, sc.pool, sc.stream) : cudaMalloc(&p, bytes);
+    }
+    void* get() const { return p; }
+    template <class T>
+    T* as() const { return static_cast<T*>(p); }
+    ~AsyncBuf() {
+        if (p && from.pool) cudaFreeAsync(p, from.stream);
+        if (p && !from.pool) cudaFree(p);
+    }
+};
+
+// Mapped host buffers (spike logs, record rows) that leaving instances give
+// back for the next ones: locking their pages took 4 ms of the 15 ms of
+// admitting a 40,000-neuron request.  Keeps at most kKeep bytes, frees them
+// with the engine's last instance; used by the admission and the stepping
+// thread.
+struct HostPool {
+    static constexpr std::size_t kKeep = 64u << 20;
+    std::mutex mu;
+    std::vector<std::pair<std::size_t, void*>> kept;
+    std::size_t held = 0;
+    static std::size_t rounded(std::size_t bytes) {
+        std::size_t r = 4096;
+        while (r < bytes) r *= 2;
+        return r;
+    }
+    cudaError_t take(std::size_t bytes, void** p);
+    void give(void* p, std::size_t bytes);
+    ~HostPool();
+};
+
 // One resident instance.
 struct Instance {
     int id = -1;
     InstDev dev{};             // host copy of the device descriptor
-    DevBuf arena;              // every device array of the instance
+    AsyncBuf arena;            // every device array of the instance
     std::size_t arena_bytes = 0;
     // Launches of several steps (see Span): the most steps this instance's
     // delays allow (1: none), their spike lists and SIC factor rows, and
     // whether the factors live there now or in the arena.
     int span_max = 1;
-    DevBuf span;
+    AsyncBuf span;
+    std::size_t span_bytes = 0;
+    std::atomic<std::uint64_t>* span_total = nullptr;  // the engine's count of them
+    void drop_span();
     double* span_fac = nullptr;
     std::uint32_t* span_fany = nullptr;
     bool fac_in_span = false;
@@ -52,6 +112,8 @@ struct Instance {
     unsigned long long* log_d[2] = {nullptr, nullptr};
     double* rec_h[2] = {nullptr, nullptr};  // Ca | IP3 | V | Isic rows
     double* rec_d[2] = {nullptr, nullptr};
+    std::shared_ptr<HostPool> host_pool;
+    std::size_t log_bytes = 0, rec_bytes = 0;
     std::uint32_t log_cap = 0;
     std::uint32_t rec_rows = 0;
     std::int64_t chunk_first[2] = {0, 0};   // first step of the chunk written to parity p
@@ -73,6 +135,7 @@ struct EngineConfig {
     int occupancy = 0;  // 0 auto, 1 latency form, 2 high-occupancy form of the step kernel
     bool large_total = false;  // the engine will hold 2^16+ neurons in all (auto SIC form)
     bool astro_fp32 = false;   // precision study: astrocyte update in FP32
+    bool keep_memory = false;  // instances come and go (a server): see Scratch
     bool item_loop = true;     // high-occupancy form: one wave, several items per block
 };
 
@@ -125,6 +188,9 @@ public:
     double chunk_device_ms = 0.0;  // sum over collected chunks (serving)
     std::int64_t launched_kernels = 0;
     std::atomic<std::uint64_t> resident_bytes{0};  // also read by a preparing thread
+    std::atomic<std::uint64_t> span_bytes{0};      // span buffers of all instances
+    std::uint64_t free_at_init = 0;
+    bool budget_given = false;  // cfg.mem_budget is the caller's, not the default
     cudaStream_t stream = nullptr;
     int sms = 148;
 
@@ -180,6 +246,11 @@ private:
     static constexpr int kSideEvents = 8;
     cudaStream_t side = nullptr;
     cudaStream_t upload = nullptr;  // table uploads of add(), beside the chunks in flight
+    cudaMemPool_t pool = nullptr;  // admission scratch (and a server's arenas)
+    int prepare_instance(const asg_network_desc& d, const asg_record_opts* rec, std::int64_t first,
+                         std::int64_t end, bool keep_spikes, bool check_budget,
+                         std::unique_ptr<Instance>* out);
+    std::shared_ptr<HostPool> host_pool = std::make_shared<HostPool>();
     std::vector<Work> side_work;
     DevBuf d_side_work;
     int side_lead = 0, side_lead_max = 0;

@@ -340,6 +340,7 @@ int asg_serve_create(const asg_serve_opts* opts, asg_server** out) {
     auto s = std::make_unique<Server>();
     asg::EngineConfig cfg = asg::config_from(opts ? &opts->engine : nullptr);
     if (opts == nullptr || opts->engine.chunk_steps <= 0) cfg.chunk_steps = 64;
+    cfg.keep_memory = true;
     s->eng = std::make_unique<asg::Engine>(cfg);
     ASG_TRY(s->eng->init());
     if (opts != nullptr && opts->mem_budget > 0) {
@@ -350,6 +351,7 @@ int asg_serve_create(const asg_serve_opts* opts, asg_server** out) {
         s->budget = static_cast<std::uint64_t>(0.8 * static_cast<double>(fr));
     }
     s->eng->cfg.mem_budget = s->budget + (1ull << 30);
+    s->eng->budget_given = opts != nullptr && opts->mem_budget > 0;
     if (opts != nullptr && opts->max_instances > 0) s->max_instances = opts->max_instances;
     Server* raw = s.get();
     s->thread = std::thread([raw] { raw->loop(); });
