@@ -860,7 +860,7 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
     // One push block per kPushCells neurons, at most two per SM: the grid
     // of a step (push, SIC parts, neurons, astrocytes) should fit the GPU in
     // one wave; a burst is spread over the blocks' threads by striding.
-    D.push_blocks = static_cast<std::int32_t>(std::min<std::uint32_t>(
+    I.step_push_blocks = static_cast<std::int32_t>(std::min<std::uint32_t>(
         2u * static_cast<std::uint32_t>(sms),
         std::max<std::uint32_t>(1, (N + kPushCells - 1) / kPushCells)));
     D.seed = d.seed;
@@ -1249,40 +1249,62 @@ int Engine::rebuild() {
         D.fany_slots = p->fac_in_span ? D.d_a2n + 2 * kMaxSpan : D.slots + 1;
         D.fany_ahead = p->fac_in_span ? kMaxSpan : 1;
     }
-    work.clear();
-    order.clear();
-    // Push and SIC blocks first (longest dependent chains), then neurons, then
-    // astrocytes.  A PUSH item's `first` is its index among the instance's
-    // push blocks.
-    std::vector<std::uint32_t> helpers(insts.size(), 0);
-    for (int role = 0; role < 4; ++role) {
-        for (std::size_t s = 0; s < insts.size(); ++s) {
-            const InstDev& D = insts[s]->dev;
-            const std::uint16_t r = role == 0   ? kRolePush
-                                    : role == 1 ? kRoleSic
-                                    : role == 2 ? kRoleNeuron
-                                                : kRoleAstro;
-            if (r == kRoleSic && (D.fused_sic || D.sic_inline || (D.sic_side && cfg.use_graphs != 2)))
-                continue;
-            if (r == kRolePush) {
-                if (!D.deferred_push) continue;
-                for (int pb = 0; pb < D.push_blocks; ++pb)
-                    work.push_back(Work{static_cast<std::uint32_t>(s), r, kNoHelper,
-                                        static_cast<std::uint32_t>(pb), 0});
-                continue;
-            }
-            const std::uint32_t n = r == kRoleAstro ? D.NA
-                                    : r == kRoleSic ? static_cast<std::uint32_t>(D.sic_parts) * D.sic_npad
-                                                    : D.N;
-            for (std::uint32_t f = 0; f < n; f += B) {
-                const std::uint16_t h = D.deferred_push && helpers[s] < kNoHelper
-                                            ? static_cast<std::uint16_t>(helpers[s]++)
-                                            : kNoHelper;
-                work.push_back(Work{static_cast<std::uint32_t>(s), r, h, f,
-                                    std::min<std::uint32_t>(B, n - f)});
+    // The work table.  Push and SIC blocks first (longest dependent chains),
+    // then neurons, then astrocytes; in the wide form of several-step launches
+    // the longest items first -- neurons, then astrocytes, which balances the
+    // blocks' last items -- and a quarter of the push blocks, last: their
+    // pushes have the whole launch's time (10^6 neurons 81.5 -> 80.4 us per step,
+    // 50,000 5.90 -> 5.63, the 64-instance sweep 7.50 -> 7.37).  A PUSH item's
+    // `first` is its index among the instance's push blocks.
+    std::vector<std::uint32_t> helpers;
+    auto fill_work = [&](bool span_wide) {
+        work.clear();
+        helpers.assign(insts.size(), 0);
+        for (int at = 0; at < 4; ++at) {
+            const int role = span_wide ? (at + 2) % 4 : at;
+            for (std::size_t s = 0; s < insts.size(); ++s) {
+                InstDev& D = insts[s]->dev;
+                const std::uint16_t r = role == 0   ? kRolePush
+                                        : role == 1 ? kRoleSic
+                                        : role == 2 ? kRoleNeuron
+                                                    : kRoleAstro;
+                if (r == kRoleSic && (D.fused_sic || D.sic_inline || (D.sic_side && cfg.use_graphs != 2)))
+                    continue;
+                if (r == kRolePush) {
+                    if (!D.deferred_push) continue;
+                    D.push_blocks = span_wide ? (insts[s]->step_push_blocks + 3) / 4
+                                              : insts[s]->step_push_blocks;
+                    for (int pb = 0; pb < D.push_blocks; ++pb)
+                        work.push_back(Work{static_cast<std::uint32_t>(s), r, kNoHelper,
+                                            static_cast<std::uint32_t>(pb), 0});
+                    continue;
+                }
+                const std::uint32_t n = r == kRoleAstro ? D.NA
+                                        : r == kRoleSic
+                                            ? static_cast<std::uint32_t>(D.sic_parts) * D.sic_npad
+                                            : D.N;
+                for (std::uint32_t f = 0; f < n; f += B) {
+                    const std::uint16_t h = D.deferred_push && helpers[s] < kNoHelper
+                                                ? static_cast<std::uint16_t>(helpers[s]++)
+                                                : kNoHelper;
+                    work.push_back(Work{static_cast<std::uint32_t>(s), r, h, f,
+                                        std::min<std::uint32_t>(B, n - f)});
+                }
             }
         }
-    }
+    };
+    fill_work(false);
+    // Step kernel form: a large step is throughput-bound and the wide form runs
+    // it faster; a smaller one is bound by its dependent round trips, which the
+    // latency form keeps fewest.  Launches of one step: the line lies at two
+    // waves of the latency form (4 blocks of 128 threads per SM).  Launches of
+    // several: a little above one wave of it (3 per SM); per step, latency and
+    // wide form: 25,000 neurons (490 items) 3.17 and 3.59 us, 30,000 (588) 4.22
+    // and 3.60, 60,000 7.47 and 6.01.
+    const std::size_t line = span > 1 ? static_cast<std::size_t>(7 * sms / 2)
+                                      : static_cast<std::size_t>(8 * sms);
+    wide = cfg.block == 128 && (cfg.occupancy == 2 || (cfg.occupancy == 0 && work.size() > line));
+    if (wide && span > 1) fill_work(true);
     for (std::size_t s = 0; s < insts.size(); ++s)
         insts[s]->dev.push_helpers = static_cast<std::int32_t>(helpers[s]);
     // Side-stream SIC batches (graph and plain launches; the persistent
@@ -1333,16 +1355,6 @@ int Engine::rebuild() {
     ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, cap_insts * kStatWords * sizeof(unsigned long long),
                              stream));
     ASG_CUDA(cudaStreamSynchronize(stream));
-    // Step kernel form: a large step is throughput-bound and the wide form runs
-    // it faster; a smaller one is bound by its dependent round trips, which the
-    // latency form keeps fewest.  Launches of one step: the line lies at two
-    // waves of the latency form (4 blocks of 128 threads per SM).  Launches of
-    // several: a little above one wave of it (3 per SM); per step, latency and
-    // wide form: 25,000 neurons (490 items) 3.17 and 3.59 us, 30,000 (588) 4.22
-    // and 3.60, 60,000 7.47 and 6.01.
-    const std::size_t line = span > 1 ? static_cast<std::size_t>(7 * sms / 2)
-                                      : static_cast<std::size_t>(8 * sms);
-    wide = cfg.block == 128 && (cfg.occupancy == 2 || (cfg.occupancy == 0 && work.size() > line));
     // The large forms run as one wave of resident blocks, each taking several
     // work items (no per-item block launch or descriptor staging after its
     // first).

@@ -91,6 +91,7 @@ struct Instance {
     // delays allow (1: none), their spike lists and SIC factor rows, and
     // whether the factors live there now or in the arena.
     int span_max = 1;
+    int step_push_blocks = 0;  // PUSH items (a quarter in the wide form of several steps)
     AsyncBuf span;
     std::size_t span_bytes = 0;
     std::atomic<std::uint64_t>* span_total = nullptr;  // the engine's count of them
@@ -230,7 +231,6 @@ private:
     int persistent_grid = 0;
     std::size_t cap_insts = 0;
     std::vector<Work> work;
-    std::vector<int> order;  // instance index per device slot
     // Captured chunk graphs by length, most recently used first: the
     // chunk_steps graph and the lengths run() splits its calls into.
     static constexpr std::size_t kMaxGraphs = 4;
