@@ -16,8 +16,9 @@ noise off).  One "step" is one timestep of all N cells.
   the movement pattern of the reference's published GPU numbers.
 - roofline: the binding one is the FP64 pipe (FP64 flops counted by ncu per
   cell-step / launch time, against 148 SMs x 64 FP64 lanes x 2 flops x the
-  sampled SM clock); the HBM roofline (48 algorithmic bytes per cell-step
-  against the measured copy bandwidth) is reported beside it.
+  sampled SM clock); the HBM roofline (48 algorithmic bytes per cell and
+  launch, a launch running all of a call's steps, against the measured copy
+  bandwidth) is reported beside it.
 - cpu_baseline: the reference's own astro_advance (built from its sources,
   oracle/_ref) over a bounded sample on the host cores with OpenMP.
 - reference_cuda_kernel: the reference's astro_update_kernel built for
@@ -55,17 +56,17 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "neuron-updates/s & HBM GB/s vs roofline; batched/served vs plain; p50/p99 lat"
-BYTES_PER_CELL_STEP = 48  # Ca, IP3, h: read + write, FP64
+BYTES_PER_CELL = 48  # Ca, IP3, h: read + write, FP64; once per launch, whatever its steps
 # Per cell-step of astro_step_kernel<uniform, bernoulli> (substeps 1), from
 # an ncu capture of the headline workload (profiles/astro_step_kernel_N1e7.md):
 # FP64 thread instructions executed (DADD + DMUL + DFMA + the rest of the
 # FP64 pipe) and FP64 flops (DFMA counted twice).
-FP64_INST_PER_CELL_STEP = 313  # 64 DADD + 109 DMUL + 134 DFMA + 6 other
-FP64_FLOP_PER_CELL_STEP = 441
+FP64_INST_PER_CELL_STEP = 297  # 64 DADD + 109 DMUL + 118 DFMA + 6 other
+FP64_FLOP_PER_CELL_STEP = 409
 FP64_LANES_PER_SM = 64
 # dram__bytes_read.sum + dram__bytes_write.sum of one astro_step_kernel launch
-# at N = 1e7, from the same capture.
-NCU_TRAFFIC_PER_LAUNCH = {10_000_000: 420_352_512}
+# (20 steps) at N = 1e7, from the same capture.
+NCU_TRAFFIC_PER_LAUNCH = {10_000_000: 420_555_264}
 
 
 def load_peaks():
@@ -229,7 +230,8 @@ def bench_astro_scaling(args, rank, world, pg):
     barrier(pg)
     step += args.steps
     dev_ms = max_over_ranks(pg, dev_ms)
-    per_launch_us = dev_ms * 1e3 / args.steps
+    per_launch_us = dev_ms * 1e3 / max(kernels, 1)  # a launch runs all of a call's steps
+    us_per_step = dev_ms * 1e3 / args.steps
     value = n * world * args.steps / (dev_ms * 1e-3)
     clocks = clk.summary()
 
@@ -270,18 +272,18 @@ def bench_astro_scaling(args, rank, world, pg):
     eng_e2e.destroy()
 
     peak, peak_kind = load_peaks()
-    achieved = BYTES_PER_CELL_STEP * n / (per_launch_us * 1e-6) / 1e9
+    achieved = BYTES_PER_CELL * n / (per_launch_us * 1e-6) / 1e9
     hbm = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
            "frac": achieved / peak, "traffic": NCU_TRAFFIC_PER_LAUNCH.get(n),
            "traffic_unit": "bytes per launch (ncu dram read + write)",
            "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
-           else peak_kind, "bytes_per_launch": BYTES_PER_CELL_STEP * n}
+           else peak_kind, "bytes_per_launch": BYTES_PER_CELL * n}
     roofline = dict(hbm)
     if FP64_FLOP_PER_CELL_STEP is not None and clocks.get("sm_mhz"):
         sms = sm_count()
         peak_tf = sms * FP64_LANES_PER_SM * 2 * clocks["sm_mhz"] * 1e6 / 1e12
-        ach_tf = FP64_FLOP_PER_CELL_STEP * n / (per_launch_us * 1e-6) / 1e12
-        inst_rate = FP64_INST_PER_CELL_STEP * n / (per_launch_us * 1e-6)
+        ach_tf = FP64_FLOP_PER_CELL_STEP * n / (us_per_step * 1e-6) / 1e12
+        inst_rate = FP64_INST_PER_CELL_STEP * n / (us_per_step * 1e-6)
         roofline = {"bound": "fp64", "achieved": ach_tf, "peak": peak_tf, "unit": "TFLOP/s",
                     "frac": ach_tf / peak_tf,
                     "fp64_pipe_inst_frac": inst_rate / (sms * FP64_LANES_PER_SM *
@@ -602,6 +604,11 @@ def run_reference_arm(args, rank, world, pg):
     from astrosimgpu_b200.astro import ScalingWorkload
 
     from oracle import ref
+    if not ref.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "no reference build (oracle/_ref) and no reference sources to make one"}),
+              flush=True)
+        return 0
     threads = os.cpu_count() or 1
     w = ScalingWorkload(args.cells)
     Ca, IP3, h = [a.copy() for a in w.initial_state()]
@@ -694,7 +701,10 @@ def main():
                 extras[key] = {"unavailable": f"{type(e).__name__}: {str(e)[:300]}"}
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cpu = cpu_baseline(w)
+        try:
+            cpu = cpu_baseline(w)
+        except OSError as e:  # the reference build is absent
+            cpu = {"unavailable": str(e)[:200]}
 
     if rank == 0:
         line = {

@@ -152,8 +152,11 @@ typedef struct asg_engine_opts {
                                ~2^23 / neurons as a power of two in [32, 512];
                                batches and servers 32 and 64)                  */
     int32_t block;          /* threads per block of the step kernel (default 128)  */
-    int32_t use_graphs;     /* 0/1 = a CUDA graph of per-step launches (default),
-                               -1 = plain launches, 2 = persistent: one cooperative
+    int32_t use_graphs;     /* 0/1 = a CUDA graph of launches (default), of several
+                               steps each where the delays allow (up to half
+                               the spike delay, at most 8), else of one;
+                               -1 = plain launches, one per step; 2 =
+                               persistent: one cooperative
                                launch per chunk, bounded grid barrier per step    */
     int32_t sic_mode;       /* 0 auto, 1 fused into the neuron role, 2 own role.
                                Auto fuses for a one-step SIC delay and, with
@@ -217,7 +220,7 @@ int asg_destroy(asg_network* net);
 
 /* ------------------------------------------------------ batched sweep
  * Many instances of uneven size packed into one device arena and advanced
- * together by one fused kernel per step, captured in CUDA graphs. */
+ * together by one fused kernel per launch, captured in CUDA graphs. */
 typedef struct asg_batch asg_batch;
 
 int asg_batch_create(int32_t n, const asg_network_desc* const* descs,
