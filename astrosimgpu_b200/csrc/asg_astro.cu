@@ -6,7 +6,8 @@
 // Layout: SoA FP64 arrays Ca, IP3, h (+ Ca_tot, IP3_0, tau_IP3, delta_IP3
 // when per-cell), 256-byte aligned.  A thread owns one, two or four adjacent
 // cells (the launch shape), read and written with coalesced accesses; one
-// thread per unit of cells, no loop over the grid.
+// thread per unit of cells, no loop over the grid.  The kernel-scaling workload
+// runs all of a call's steps in one launch.
 //
 // Compiled with -fmad=false: results are bitwise equal to the host's
 // astro_advance (no transcendental on this path when noise is off).

@@ -351,8 +351,9 @@ __device__ __forceinline__ AstroRates li_rinzel(const AstroK& k, double ca_tot, 
 // side in the instruction stream, for kernels that also hold other roles'
 // code); the weighted stage sum is accumulated left to right either way, so
 // both forms perform the same IEEE operations in the same order.
-// kNewton = false divides with the compiler's IEEE division (the network step
-// kernels, whose other roles it slows: use_case 3.43 -> 3.63 us per step).
+// kNewton = false divides with the compiler's IEEE division (the kernels
+// of single network steps, whose other roles it slows: use_case 3.43 -> 3.63 us
+// per step; the kernels of several steps per launch use div_newton).
 template <bool kUnroll = true, bool kNewton = true>
 __device__ __forceinline__ void astro_rk4(const AstroK& k, double ca_tot, double ip3_0, double tau,
                                           double inv_tau, double delta, double input, double noise,

@@ -227,7 +227,7 @@ struct InstDev {
 // round trip are paid once per launch instead of once per step.  With delays
 // of ten steps (five per launch), per step: 500 neurons 3.32 -> 2.05 us (a step
 // is now its RK4 chain, ~1.1 us, the rest of its loop and a fifth of a launch
-// boundary), 10,000 4.1 -> 2.5, 200,000 25.8 -> 19.2, 10^6 118 -> 82.
+// boundary), 10,000 4.1 -> 2.4, 200,000 25.8 -> 18.8, 10^6 118 -> 80.
 //
 // Spike lists: list 3 is the arena's, by step (the launches of one step);
 // 0..2 are span headers i % 3 with the records in span list i & 1.  A chunk of

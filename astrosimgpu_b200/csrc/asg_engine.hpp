@@ -1,7 +1,8 @@
 // Host side of the network engine: one Engine holds any number of resident
 // network instances (a plain run is an engine with one instance, a sweep is
 // a batch, serving adds and removes instances at step boundaries) and
-// advances them together, one fused kernel launch per step, K steps per
+// advances them together, one fused kernel launch per step or per several
+// steps (Span in asg_engine.cuh), K steps per
 // captured CUDA graph ("chunk").
 #pragma once
 

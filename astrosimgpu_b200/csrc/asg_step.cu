@@ -1,5 +1,5 @@
-// The fused per-timestep kernel of the network engine (layout and design in
-// asg_engine.cuh).  Compiled with -fmad=false: every floating-point
+// The fused step kernels of the network engine (layout and design in
+// asg_engine.cuh; launches of several steps: Span there).  Compiled with -fmad=false: every floating-point
 // expression is evaluated as separate IEEE operations in the reference's
 // order (neuron.cpp:101-250, astrocyte.cpp:233-329, network.cpp:230-355).
 //
