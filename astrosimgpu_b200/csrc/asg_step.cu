@@ -1637,72 +1637,63 @@ __global__ void __launch_bounds__(kMaxBlock) chunk_kernel(const InstDev* __restr
     }
 }
 
-// Side-stream SIC batch: thread per target, its whole list (P = 1), and the
-// sums of all kSicBatchSteps arrival steps of the batch at once: for each
-// list entry the factors of the astrocyte at the arrivals' emission steps
-// are loaded together, and the m additions of the entry advance the
-// kSicBatchSteps sums side by side -- independent chains, each the SIC
-// role's sequential sum (a zero factor adds +0.0, exact since a sum that
-// starts at +0.0 and adds nonzero values is never -0.0).  One block per
-// work item, so the batch leaves the SMs to the step kernels beside it.
+// Side-stream SIC batch: a thread per target and arrival step (blockIdx.y) of
+// the batch sums the target's whole list (P = 1), the SIC role's sequential sum:
+// the factors of kSicBatch entries and the entries after them are loaded
+// together, then each entry's factor is added m times (a zero factor adds
+// +0.0, exact since a sum that starts at +0.0 and adds nonzero values is never
+// -0.0).
 // Launched when the step before step0+k has completed (the factors it
-// needs are older still), and waited for before the first step that reads it.
+// needs are older still), and waited for before the first step that reads it:
+// a batch that takes longer than the launches beside it is what the steps wait
+// for.  One thread with the chains of all eight arrivals took that long (10,000
+// targets of ~400 edges: 79 blocks, 30 us alone -- a round trip per entry's
+// factors, sixteen 64-bit remainders one after another, eight additions per
+// edge); a thread per arrival takes 14 us alone.  Per paper_sparse_dt005 step,
+// quiet / every astrocyte emitting / over 1 s: 3.11 / 3.78 / 3.76 -> 2.28 /
+// 3.43 / 3.25 us (two arrivals per thread: 2.59 / 3.52 / 3.42).
 __global__ void __launch_bounds__(kMaxBlock) sic_batch_kernel(const InstDev* __restrict__ insts,
                                                               const Work* __restrict__ work,
                                                               int k) {
-    constexpr int G = kSicBatchSteps;
     const Work wk = load_work(work + blockIdx.x);
     const InstDev& I = insts[wk.inst];
+    const std::int64_t a = I.step0 + k + I.sic_lead + static_cast<int>(blockIdx.y);
+    const std::int64_t se = a - I.d_a2n;
+    const bool due = a >= I.step0 && se >= 0 && se % I.sic_interval == 0;
     unsigned long long edges = 0;
-    if (threadIdx.x < wk.count) {
+    if (due && threadIdx.x < wk.count) {
         const std::uint32_t t = wk.first + threadIdx.x;
         std::uint32_t o0 = 0, len = 0, e[kSicBatch];
         sic_prefetch(I, t, o0, len, e);
-        const double* fac[G];
-        bool due[G];
-        double acc[G];
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-            const std::int64_t a = I.step0 + k + I.sic_lead + j;
-            const std::int64_t se = a - I.d_a2n;
-            due[j] = a >= I.step0 && se >= 0 && se % I.sic_interval == 0;
-            fac[j] = I.fac + static_cast<std::size_t>(due[j] ? se % I.fac_slots : 0) * I.NA;
-            acc[j] = 0.0;
-        }
+        const double* fac = I.fac + static_cast<std::size_t>(se % I.fac_slots) * I.NA;
+        double acc = 0.0;
         for (std::uint32_t b0 = 0;; b0 += kSicBatch) {
-            bool done = false;
-            for (int q = 0; q < kSicBatch; ++q) {
-                const std::uint32_t m = e[q] & 0xFFu;
-                if (m == 0) {
-                    done = true;  // padding ends the list
-                    break;
-                }
-                const std::uint32_t as = e[q] >> 8;
-                double c[G];
-#pragma unroll
-                for (int j = 0; j < G; ++j) {
-                    const double f = __ldcg(fac[j] + as);
-                    c[j] = I.w_a2n * f;
-                    if (due[j] && f != 0.0) edges += m;
-                    if (f == 0.0) c[j] = 0.0;
-                }
-                for (std::uint32_t r = 0; r < m; ++r) {
-#pragma unroll
-                    for (int j = 0; j < G; ++j) acc[j] += c[j];
-                }
-            }
-            if (done || b0 + kSicBatch >= len) break;
+            // Padding entries read astrocyte 0 and add nothing.
+            double f[kSicBatch];
+            std::uint32_t m[kSicBatch];
 #pragma unroll
             for (int q = 0; q < kSicBatch; ++q) {
-                const std::uint32_t jj = b0 + kSicBatch + q;
-                e[q] = jj < len ? __ldg(I.sic_ent + o0 + jj * 32) : 0u;
+                m[q] = e[q] & 0xFFu;
+                f[q] = __ldcg(fac + (e[q] >> 8));
             }
-        }
+            const bool last = m[kSicBatch - 1] == 0 || b0 + kSicBatch >= len;
+            if (!last) {
 #pragma unroll
-        for (int j = 0; j < G; ++j) {
-            const std::int64_t a = I.step0 + k + I.sic_lead + j;
-            if (due[j]) I.sic_val[static_cast<std::size_t>(a & (I.sic_ring - 1)) * I.N + t] = acc[j];
+                for (int q = 0; q < kSicBatch; ++q) {
+                    const std::uint32_t jj = b0 + kSicBatch + q;
+                    e[q] = jj < len ? __ldg(I.sic_ent + o0 + jj * 32) : 0u;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kSicBatch; ++q) {
+                const std::uint32_t n = f[q] == 0.0 ? 0u : m[q];
+                const double c = I.w_a2n * f[q];
+                edges += n;
+                for (std::uint32_t r = 0; r < n; ++r) acc += c;
+            }
+            if (last) break;
         }
+        I.sic_val[static_cast<std::size_t>(a & (I.sic_ring - 1)) * I.N + t] = acc;
     }
     for (int o = 16; o > 0; o >>= 1) edges += __shfl_down_sync(0xFFFFFFFFu, edges, o);
     if ((threadIdx.x & 31) == 0 && edges) atomicAdd(I.counters + 1, edges);
@@ -1719,7 +1710,8 @@ __global__ void barrier_selftest_kernel(GridBarrier* gb) {
 
 cudaError_t launch_sic_batch(const InstDev* insts, const Work* work, int n_work, int block, int k,
                              cudaStream_t stream) {
-    sic_batch_kernel<<<static_cast<unsigned>(n_work), block, 0, stream>>>(insts, work, k);
+    const dim3 grid(static_cast<unsigned>(n_work), kSicBatchSteps);
+    sic_batch_kernel<<<grid, block, 0, stream>>>(insts, work, k);
     return cudaGetLastError();
 }
 
