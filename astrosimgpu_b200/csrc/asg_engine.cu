@@ -3,6 +3,7 @@
 // the work table, captured chunks and output collection.
 
 #include "asg_engine.hpp"
+#include "asg_span.hpp"
 
 #include <cub/cub.cuh>
 
@@ -953,13 +954,19 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
         } else if (NA > 0) {
             L = D.sic_parts > 1 ? 1 : std::min(L, D.d_a2n - (D.fused_sic ? 0 : 1));
         }
+        std::uint64_t edges = 0;
         for (const asg_csr* c : {&d.exc_primary, &d.inh_primary, &d.neuron_astro}) {
             const std::uint32_t* rs = rs_of(*c);  // a spike record holds a row length in 28 bits
+            edges += rs[c->n_sources];
             if (first_bad(c->n_sources, [&](std::uint32_t i) {
                     return rs[i + 1] - rs[i] >= (1u << 28);
                 }) < c->n_sources)
                 L = 1;
         }
+        const int ref = NE == 0 ? D.pi.ref_steps
+                        : NI == 0 ? D.pe.ref_steps
+                                  : std::min(D.pe.ref_steps, D.pi.ref_steps);
+        L = span_that_fits(L, N, edges, d.substeps, ref);
         I.span_max = std::max(1, L);
     }
     SicHost sic;
