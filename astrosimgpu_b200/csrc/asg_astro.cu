@@ -328,11 +328,15 @@ cudaError_t launch_update(bool uniform, bool pending, bool noisy, int shape,
                    : launch_update_p<false>(pending, noisy, shape, a, s, st);
 }
 
-// Steps of the Bernoulli workload per launch: all of a call's, up to 2^33
-// cell-steps (about 0.2 s), which bounds a launch's length.
-int steps_per_launch(std::int64_t n, std::int64_t left) {
-    return static_cast<int>(std::min<std::int64_t>(
-        left, std::max<std::int64_t>(1, std::min<std::int64_t>((1ll << 33) / n, 1 << 30))));
+// Steps of the Bernoulli workload per launch: all of a call's, up to a launch of
+// about 0.2 s.  A large population is bound by its work, 2^33 cell-substeps at
+// 5e10 per second; a small one by the chain of a thread's substeps, 2^17 of
+// them at 0.7 us (a thread of several cells takes up to three times as long).
+int steps_per_launch(std::int64_t n, int substeps, std::int64_t left) {
+    const std::int64_t sub = std::max(1, substeps);
+    const std::int64_t work = (std::int64_t{1} << 33) / std::max<std::int64_t>(1, n) / sub;
+    const std::int64_t chain = (std::int64_t{1} << 17) / sub;
+    return static_cast<int>(std::min(left, std::max<std::int64_t>(1, std::min(work, chain))));
 }
 
 // ceil(p * 2^53): k * 2^-53 < p exactly when the integer k is below it
@@ -748,7 +752,7 @@ int asg_astro_run_bernoulli(asg_astro* s, const double* consts, double h_step, i
     std::int64_t kernels = 0;
     for (std::int64_t done = 0; done < count; ++kernels) {
         a.step0 = first + done;
-        a.n_steps = asg::steps_per_launch(e->n, count - done);
+        a.n_steps = asg::steps_per_launch(e->n, substeps, count - done);
         ASG_CUDA((uniform ? asg::launch_astro<true, asg::kInputBernoulli, false>(
                                 e->shape, a, e->arrays(), e->stream)
                           : asg::launch_astro<false, asg::kInputBernoulli, false>(
@@ -830,7 +834,7 @@ int asg_astro_run_bernoulli_f32(asg_astro* s, const double* consts, double h_ste
     std::int64_t kernels = 0;
     for (std::int64_t done = 0; done < count; ++kernels) {
         a.step0 = first + done;
-        a.n_steps = asg::steps_per_launch(e->n, count - done);
+        a.n_steps = asg::steps_per_launch(e->n, substeps, count - done);
         asg::astro_step_kernel_f32<<<grid, 128, 0, e->stream>>>(
             a, kf, e->Ca32.as<float>(), e->IP332.as<float>(), e->h32.as<float>());
         ASG_CUDA(cudaGetLastError());
@@ -902,7 +906,7 @@ extern "C" int asg_astro_autotune(asg_astro* s, const double* consts, double h_s
             ASG_CUDA(cudaEventRecord(e->ev0, e->stream));
             for (int done = 0; done < steps; done += a.n_steps) {
                 a.step0 = done;
-                a.n_steps = asg::steps_per_launch(e->n, steps - done);
+                a.n_steps = asg::steps_per_launch(e->n, substeps, steps - done);
                 ASG_CUDA((asg::launch_astro<true, asg::kInputBernoulli, false>(shape, a,
                                                                                 arr, e->stream)));
             }
