@@ -538,13 +538,7 @@ std::size_t align256(std::size_t x) { return (x + 255) & ~static_cast<std::size_
 
 }  // namespace
 
-void Instance::drop_span() {
-    if (span_total) span_total->fetch_sub(span_bytes);
-    span_total = nullptr;
-}
-
 Instance::~Instance() {
-    drop_span();
     for (int p = 0; p < 2; ++p) {
         if (log_h[p]) host_pool->give(log_h[p], log_bytes);
         if (rec_h[p]) host_pool->give(rec_h[p], rec_bytes);
@@ -623,12 +617,11 @@ int Engine::init() {
     if (cfg.block <= 0) cfg.block = 128;
     if (cfg.block > 512 || cfg.block % 32 != 0)
         return fail(ASG_ERR_ARG, "block size %d must be a multiple of 32 in [32, 512]", cfg.block);
-    std::size_t fr = 0, tot = 0;
-    ASG_CUDA(cudaMemGetInfo(&fr, &tot));
-    free_at_init = fr;
-    budget_given = cfg.mem_budget != 0;
-    if (cfg.mem_budget == 0)
+    if (cfg.mem_budget == 0) {
+        std::size_t fr = 0, tot = 0;
+        ASG_CUDA(cudaMemGetInfo(&fr, &tot));
         cfg.mem_budget = static_cast<std::uint64_t>(0.9 * static_cast<double>(fr));
+    }
     ASG_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     ASG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     ASG_CUDA(cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking));
@@ -1108,38 +1101,6 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
         ASG_CUDA(cudaStreamSynchronize(upload));  // host sources go out of scope
     }
 
-    // The span buffers stay within a budget the caller gave; beside the default
-    // one they take at most half of what it leaves free.  Without one the
-    // instance runs one step per launch.
-    if (I.span_max > 1) {
-        const std::size_t cap = static_cast<std::size_t>(N) * I.span_max;
-        const std::size_t rec = align256(2 * cap * 16);
-        const std::size_t fac = D.sic_side ? 0 : align256(static_cast<std::size_t>(D.d_a2n + kMaxSpan) * a8);
-        const std::size_t any = align256((static_cast<std::size_t>(D.d_a2n) + 2 * kMaxSpan) * 4);
-        const std::size_t bytes = 2 * rec + fac + any;
-        const std::uint64_t spans = span_bytes.fetch_add(bytes) + bytes;
-        const std::uint64_t spare =
-            free_at_init > cfg.mem_budget ? (free_at_init - cfg.mem_budget) / 2 : 0;
-        const bool room = budget_given ? resident_bytes + total + spans <= cfg.mem_budget
-                                       : spans <= spare;
-        I.span_bytes = bytes;
-        I.span_total = &span_bytes;
-        if (room && need(I.span, bytes, keep) == ASG_OK) {
-            char* p = I.span.as<char>();
-            ASG_CUDA(cudaMemsetAsync(p + 2 * rec, 0, fac + any, upload));
-            ASG_CUDA(cudaStreamSynchronize(upload));
-            D.span_meta = reinterpret_cast<std::uint32_t*>(p);
-            D.span_val = reinterpret_cast<double*>(p + rec);
-            D.span_cap = cap;
-            I.span_fac = reinterpret_cast<double*>(p + 2 * rec);
-            I.span_fany = reinterpret_cast<std::uint32_t*>(p + 2 * rec + fac);
-        } else {
-            clear_error();
-            I.drop_span();
-            I.span_max = 1;
-        }
-    }
-
     // Recording and spike-log buffers (mapped host memory, two parities).
     asg_record_opts ro{};
     if (rec) ro = *rec;
@@ -1226,6 +1187,58 @@ int Engine::set_chunk(int chunk) {
     return ASG_OK;
 }
 
+// Takes the span buffers that instances lack, within the memory budget: they
+// never take room from an arena.  ASG_ERR_OOM: no room (also for those held,
+// when arenas have grown since), the engine runs one step per launch and gives
+// them back.
+int Engine::hold_span_buffers() {
+    struct Part {
+        Instance* inst;
+        std::size_t cap, rec, fac, any;
+        std::size_t bytes() const { return 2 * rec + fac + any; }
+    };
+    std::vector<Part> parts;
+    std::uint64_t want = 0;
+    for (auto& p : insts) {
+        if (p->span) continue;
+        const InstDev& D = p->dev;
+        Part q{p.get(), static_cast<std::size_t>(D.N) * p->span_max, 0, 0, 0};
+        q.rec = align256(2 * q.cap * 16);
+        q.fac = D.sic_side ? 0 : align256(static_cast<std::size_t>(D.d_a2n + kMaxSpan) * D.NA * 8);
+        q.any = align256((static_cast<std::size_t>(D.d_a2n) + 2 * kMaxSpan) * 4);
+        want += q.bytes();
+        parts.push_back(q);
+    }
+    const std::uint64_t arenas = std::max<std::uint64_t>(resident_bytes, claimed_bytes);
+    if (arenas + span_bytes + want > cfg.mem_budget)
+        return fail(ASG_ERR_OOM, "no room for the buffers of several steps per launch");
+    // One allocation for all that were added together; a server's instances
+    // leave one by one, so there each has its own, from the pool.
+    std::shared_ptr<SpanBlock> block;
+    std::size_t at = 0;
+    for (const Part& q : parts) {
+        if (cfg.keep_memory || !block) {
+            const std::uint64_t bytes = cfg.keep_memory ? q.bytes() : want;
+            block = std::make_shared<SpanBlock>(bytes, span_bytes);
+            ASG_TRY(need(block->buf, bytes, Scratch{stream, cfg.keep_memory ? pool : nullptr}));
+            at = 0;
+        }
+        char* p = block->buf.as<char>() + at;
+        at += q.bytes();
+        ASG_CUDA(cudaMemsetAsync(p + 2 * q.rec, 0, q.fac + q.any, stream));
+        InstDev& D = q.inst->dev;
+        D.span_meta = reinterpret_cast<std::uint32_t*>(p);
+        D.span_val = reinterpret_cast<double*>(p + q.rec);
+        D.span_cap = q.cap;
+        q.inst->span_fac = reinterpret_cast<double*>(p + 2 * q.rec);
+        q.inst->span_fany = reinterpret_cast<std::uint32_t*>(p + 2 * q.rec + q.fac);
+        q.inst->span = block;
+    }
+    // copy_factors writes some of it from the host's default stream
+    if (!parts.empty()) ASG_CUDA(cudaStreamSynchronize(stream));
+    return ASG_OK;
+}
+
 int Engine::rebuild() {
     ASG_TRY(finish_pending());
     ASG_CUDA(cudaStreamSynchronize(stream));
@@ -1241,6 +1254,14 @@ int Engine::rebuild() {
     }
     if (any_side)  // a divisor of the side batch
         while (kSicBatchSteps % span != 0) --span;
+    if (span > 1) {
+        const int st = hold_span_buffers();
+        if (st != ASG_OK && st != ASG_ERR_OOM) return st;
+        if (st == ASG_ERR_OOM) {
+            clear_error();
+            span = 1;
+        }
+    }
     for (auto& p : insts) {
         InstDev& D = p->dev;
         D.sic_inline = span > 1 && !D.fused_sic && !D.sic_side;
@@ -1255,6 +1276,7 @@ int Engine::rebuild() {
         D.fac_slots = p->fac_in_span ? D.d_a2n + kMaxSpan : D.slots;
         D.fany_slots = p->fac_in_span ? D.d_a2n + 2 * kMaxSpan : D.slots + 1;
         D.fany_ahead = p->fac_in_span ? kMaxSpan : 1;
+        if (span == 1) p->span.reset();
     }
     // The work table.  Push and SIC blocks first (longest dependent chains),
     // then neurons, then astrocytes; in the wide form of several-step launches

@@ -82,6 +82,16 @@ struct HostPool {
     ~HostPool();
 };
 
+// Device memory of the buffers that launches of several steps need beside the
+// arenas, of one or more instances; counted in the engine's total while held.
+struct SpanBlock {
+    AsyncBuf buf;
+    std::uint64_t bytes;
+    std::atomic<std::uint64_t>& total;
+    SpanBlock(std::uint64_t b, std::atomic<std::uint64_t>& t) : bytes(b), total(t) { total += bytes; }
+    ~SpanBlock() { total -= bytes; }
+};
+
 // One resident instance.
 struct Instance {
     int id = -1;
@@ -89,14 +99,12 @@ struct Instance {
     AsyncBuf arena;            // every device array of the instance
     std::size_t arena_bytes = 0;
     // Launches of several steps (see Span): the most steps this instance's
-    // delays allow (1: none), their spike lists and SIC factor rows, and
-    // whether the factors live there now or in the arena.
+    // delays allow (1: none), the spike lists and SIC factor rows they use,
+    // held while the engine runs them, and whether the factors live there now
+    // or in the arena.
     int span_max = 1;
     int step_push_blocks = 0;  // PUSH items (a quarter in the wide form of several steps)
-    AsyncBuf span;
-    std::size_t span_bytes = 0;
-    std::atomic<std::uint64_t>* span_total = nullptr;  // the engine's count of them
-    void drop_span();
+    std::shared_ptr<SpanBlock> span;
     double* span_fac = nullptr;
     std::uint32_t* span_fany = nullptr;
     bool fac_in_span = false;
@@ -189,10 +197,13 @@ public:
     std::int64_t chunks = 0;
     double chunk_device_ms = 0.0;  // sum over collected chunks (serving)
     std::int64_t launched_kernels = 0;
-    std::atomic<std::uint64_t> resident_bytes{0};  // also read by a preparing thread
+    std::atomic<std::uint64_t> resident_bytes{0};  // arenas; also read by a preparing thread
     std::atomic<std::uint64_t> span_bytes{0};      // span buffers of all instances
-    std::uint64_t free_at_init = 0;
-    bool budget_given = false;  // cfg.mem_budget is the caller's, not the default
+    // Bytes a server has promised to its requests, admitted or being admitted:
+    // span buffers stay out of them.
+    std::atomic<std::uint64_t> claimed_bytes{0};
+    // The next chunk decides again whether the span buffers have room.
+    void review_spans() { dirty = true; }
     cudaStream_t stream = nullptr;
     int sms = 148;
 
@@ -215,6 +226,7 @@ private:
     std::vector<Span> plan(int steps) const;  // the launches of a chunk
     cudaError_t issue_steps(int steps);  // step launches + side-stream SIC batches
     int copy_factors(Instance& I, bool to_span);
+    int hold_span_buffers();
     int span = 1;  // most steps per launch
     int launch_chunk(int parity, int steps);
     int collect(int parity);

@@ -130,11 +130,14 @@ struct Server {
     std::uint64_t resident_bytes = 0;    // footprints of running requests
     std::uint64_t reserved_bytes = 0;    // footprints of requests in admission
     std::int64_t retirements = 0;        // bumps whenever device memory frees up
+    bool spans_in_way = false;           // the request in admission waits for span buffers
     std::thread thread, admit_thread;
 
     void loop();
     void admit_loop();
     void retire(Request& r, int status);
+    // After a change of the footprints (under the lock).
+    void tell_engine() { eng->claimed_bytes = resident_bytes + reserved_bytes; }
 };
 
 void Server::retire(Request& r, int status) {
@@ -152,6 +155,7 @@ void Server::retire(Request& r, int status) {
                                     : 0.0;
         if (r.keep_spikes) r.spikes.swap(I->spikes);
         resident_bytes -= r.footprint;
+        tell_engine();
         eng->remove(r.inst);
         --resident;
         ++retirements;
@@ -193,10 +197,26 @@ void Server::admit_loop() {
             cv_admit.wait(lk, [&] { return stop || retirements != seen || r.cancel; });
             continue;
         }
-        queue.pop_front();
-        r.state = ReqState::Preparing;
         reserved_bytes += r.footprint;
         ++in_admission;
+        tell_engine();
+        // It fits, but not beside the buffers of several steps per launch: the
+        // stepping loop gives them back at its next chunk boundary.
+        auto room = [&] { return resident_bytes + reserved_bytes + eng->span_bytes <= budget; };
+        if (!room()) {
+            spans_in_way = true;
+            cv_work.notify_one();
+            cv_admit.wait(lk, [&] { return stop || r.cancel || room(); });
+            spans_in_way = false;
+            if (stop || r.cancel) {
+                reserved_bytes -= r.footprint;
+                --in_admission;
+                tell_engine();
+                continue;
+            }
+        }
+        queue.pop_front();
+        r.state = ReqState::Preparing;
         const std::int64_t seen = retirements;
         const asg_network_desc* d = &r.desc->d;
         lk.unlock();
@@ -211,6 +231,7 @@ void Server::admit_loop() {
             inst.reset();
             reserved_bytes -= r.footprint;
             --in_admission;
+            tell_engine();
             retire(r, loop_status != ASG_OK ? loop_status : ASG_ERR_CANCELLED);
             cv_done.notify_all();
             break;
@@ -220,6 +241,7 @@ void Server::admit_loop() {
             inst.reset();
             reserved_bytes -= r.footprint;
             --in_admission;
+            tell_engine();
             r.state = ReqState::Queued;
             queue.push_front(r.id);
             cv_admit.wait(lk, [&] { return stop || retirements != seen || r.cancel; });
@@ -228,6 +250,7 @@ void Server::admit_loop() {
         if (st != ASG_OK) {
             reserved_bytes -= r.footprint;
             --in_admission;
+            tell_engine();
             r.error = err;
             retire(r, st);
             cv_done.notify_all();
@@ -256,9 +279,9 @@ void Server::loop() {
         while (!staged.empty()) {
             Request& r = *reqs[staged.front()];
             staged.pop_front();
-            reserved_bytes -= r.footprint;
-            --in_admission;
             if (r.cancel) {
+                reserved_bytes -= r.footprint;
+                --in_admission;
                 retire(r, ASG_ERR_CANCELLED);
                 continue;
             }
@@ -278,6 +301,8 @@ void Server::loop() {
             lk.lock();
             for (std::size_t k = 0; k < joining.size(); ++k) {
                 Request& r = *joining[k];
+                reserved_bytes -= r.footprint;  // resident from here on
+                --in_admission;
                 if (sts[k] != ASG_OK) {
                     r.error = errs[k];
                     retire(r, sts[k]);
@@ -295,6 +320,8 @@ void Server::loop() {
             cv_work.wait(lk, [&] { return stop || !staged.empty(); });
             continue;
         }
+        tell_engine();
+        if (spans_in_way) eng->review_spans();
         // one chunk for every resident request, outside the lock
         lk.unlock();
         int st = eng->run_chunk(eng->cfg.chunk_steps);
@@ -303,6 +330,7 @@ void Server::loop() {
         // retiring requests need the outputs of every chunk still in flight
         if (st == ASG_OK && finishing) st = eng->flush();
         lk.lock();
+        if (spans_in_way) cv_admit.notify_all();
         if (st != ASG_OK) {
             loop_status = st;
             loop_error = asg_last_error();
@@ -350,8 +378,7 @@ int asg_serve_create(const asg_serve_opts* opts, asg_server** out) {
         ASG_CUDA(cudaMemGetInfo(&fr, &tot));
         s->budget = static_cast<std::uint64_t>(0.8 * static_cast<double>(fr));
     }
-    s->eng->cfg.mem_budget = s->budget + (1ull << 30);
-    s->eng->budget_given = opts != nullptr && opts->mem_budget > 0;
+    s->eng->cfg.mem_budget = s->budget;
     if (opts != nullptr && opts->max_instances > 0) s->max_instances = opts->max_instances;
     Server* raw = s.get();
     s->thread = std::thread([raw] { raw->loop(); });

@@ -168,7 +168,9 @@ typedef struct asg_engine_opts {
     int32_t push_mode;      /* 0 = spikes pushed one step later by load-balanced
                                push blocks when both spike delays are >= 2 steps
                                (default), 1 = pushed by the spiking block      */
-    uint64_t mem_budget;    /* device bytes the engine may hold (0 = 90% free)     */
+    uint64_t mem_budget;    /* device bytes the instances may hold, arenas and the
+                               buffers of launches of several steps; without room
+                               for the latter one step per launch (0 = 90% free) */
     int32_t occupancy;      /* step kernel form: 0 auto (by the number of blocks
                                a step launches), 1 latency form (fewest round
                                trips, 128 registers), 2 high-occupancy form
