@@ -92,6 +92,8 @@ int need(AsyncBuf& buf, std::size_t bytes, const Scratch& sc) {
 // the device path's launches and synchronisations take).
 constexpr std::uint32_t kDeviceEdges = 1u << 16;
 
+constexpr std::uint64_t kPoolKeep = 2ull << 30;  // unused memory a pool keeps at most
+
 struct SetTargets {
     AsyncBuf tg;             // [m], empty for a smaller set
     std::uint32_t bad = ~0u; // first edge whose target is out of range
@@ -630,8 +632,7 @@ int Engine::init() {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = cfg.device;
     ASG_CUDA(cudaMemPoolCreate(&pool, &props));
-    std::uint64_t keep = 2ull << 30;  // unused memory held
-    ASG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    claim(0);
     ASG_CUDA(cudaEventCreateWithFlags(&ev_side_fork, cudaEventDisableTiming));
     ASG_CUDA(cudaEventCreateWithFlags(&ev_side_join, cudaEventDisableTiming));
     for (int q = 0; q < kSideEvents; ++q) {
@@ -648,6 +649,17 @@ int Engine::init() {
     }
     ASG_TRY(d_barrier.alloc(sizeof(GridBarrier)));
     return ASG_OK;
+}
+
+// The pool's release threshold counts all that it holds, used or not: below
+// what the requests use, every synchronisation would give the unused memory
+// back and the next admission map it again.
+void Engine::claim(std::uint64_t bytes) {
+    claimed_bytes = bytes;
+    const std::uint64_t used = bytes + span_bytes;
+    std::uint64_t hold = used + kPoolKeep;
+    if (cfg.keep_memory) hold = std::min(hold, std::max(used, cfg.mem_budget));
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &hold);
 }
 
 Instance* Engine::find(int id) {

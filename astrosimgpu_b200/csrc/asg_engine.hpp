@@ -31,9 +31,10 @@ struct SpikeRec {
 // own.  (The default pool gives its memory back at every synchronisation and
 // the next allocation maps it again; cudaMalloc and cudaFree wait for the
 // device and, beside running chunks, took from 0.4 to tens of ms each.)  A
-// server's pool also holds the arenas and keeps up to 2 GB between requests;
-// other engines trim it after each admission and take their arenas, which
-// stay, from cudaMalloc (pool = nullptr).
+// server's pool also holds the arenas and keeps up to 2 GB beside them, within
+// the memory budget, between requests (Engine::claim); other engines trim it
+// after each admission and take their arenas, which stay, from cudaMalloc
+// (pool = nullptr).
 struct Scratch {
     cudaStream_t stream;
     cudaMemPool_t pool;
@@ -200,7 +201,8 @@ public:
     std::atomic<std::uint64_t> resident_bytes{0};  // arenas; also read by a preparing thread
     std::atomic<std::uint64_t> span_bytes{0};      // span buffers of all instances
     // Bytes a server has promised to its requests, admitted or being admitted:
-    // span buffers stay out of them.
+    // span buffers stay out of them, and the pool keeps what it needs for more.
+    void claim(std::uint64_t bytes);
     std::atomic<std::uint64_t> claimed_bytes{0};
     // The next chunk decides again whether the span buffers have room.
     void review_spans() { dirty = true; }

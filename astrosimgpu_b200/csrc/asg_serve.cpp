@@ -137,7 +137,7 @@ struct Server {
     void admit_loop();
     void retire(Request& r, int status);
     // After a change of the footprints (under the lock).
-    void tell_engine() { eng->claimed_bytes = resident_bytes + reserved_bytes; }
+    void tell_engine() { eng->claim(resident_bytes + reserved_bytes); }
 };
 
 void Server::retire(Request& r, int status) {
@@ -379,6 +379,7 @@ int asg_serve_create(const asg_serve_opts* opts, asg_server** out) {
         s->budget = static_cast<std::uint64_t>(0.8 * static_cast<double>(fr));
     }
     s->eng->cfg.mem_budget = s->budget;
+    s->eng->claim(0);
     if (opts != nullptr && opts->max_instances > 0) s->max_instances = opts->max_instances;
     Server* raw = s.get();
     s->thread = std::thread([raw] { raw->loop(); });

@@ -65,12 +65,12 @@ def test_a_request_is_admitted_beside_the_buffers_of_a_running_one():
         Server(mem_budget=1).submit(a, 10)
     need = int(re.search(r"needs ~(\d+) device bytes", str(e.value)).group(1))
     alone = []
-    for m, n in ((a, 6000), (b, 500)):
+    for m, n in ((a, 40_000), (b, 500)):
         net = Network(m)
         net.step(n)
         alone.append(net.fetch_spikes())
     s = Server(mem_budget=2 * need + (1 << 20))
-    i = s.submit(a, 6000)
+    i = s.submit(a, 40_000)
     while s.stats()["chunks"] < 4:
         time.sleep(0.001)
     first = s.stats()
@@ -82,3 +82,53 @@ def test_a_request_is_admitted_beside_the_buffers_of_a_running_one():
             assert np.array_equal(x, y)
     assert s.stats()["peak_resident"] == 2
     s.close()
+
+
+def arena_of(m):
+    net = Network(m)
+    size = len(net.checkpoint()) - 8
+    net.close()
+    return size
+
+
+def test_a_server_keeps_memory_beside_large_requests():
+    """What a request leaves stays with the server's pool for the next one (at
+    most 2 GB), also where the requests that run on hold more than that."""
+    import torch
+    m, small = serving(150_000, 4), serving(20_000, 5)
+    assert arena_of(m) > (2 << 30)
+    before = torch.cuda.mem_get_info()[0]
+
+    def held():
+        return before - torch.cuda.mem_get_info()[0]
+
+    s = Server()
+    i = s.submit(m, 200_000)
+    while s.stats()["chunks"] < 4:
+        time.sleep(0.001)
+    s.wait(s.submit(small, 64))
+    with_small, least = held(), 1 << 60
+    for _ in range(4):
+        j = s.submit(small, 64)
+        while not s.poll(j)[0]:
+            least = min(least, held())
+    s.cancel(i)
+    s.wait(i)
+    s.close()
+    assert least > with_small - (64 << 20), (least, with_small)
+
+
+def test_a_server_keeps_no_more_than_its_budget():
+    import torch
+    m = serving(20_000, 5)
+    arena = arena_of(m)
+    before = torch.cuda.mem_get_info()[0]
+    with pytest.raises(_lib.AsgError) as e:
+        Server(mem_budget=1).submit(m, 10)
+    need = int(re.search(r"needs ~(\d+) device bytes", str(e.value)).group(1))
+    small = Server(mem_budget=need)
+    assert small.wait(small.submit(m, 100)).status == 0
+    torch.cuda.synchronize()
+    held = before - torch.cuda.mem_get_info()[0]
+    small.close()
+    assert held < need + (48 << 20), (held, need, arena)
