@@ -40,6 +40,15 @@ bool injected_alloc_failure() {
     return g_alloc_count.fetch_add(1) >= limit;
 }
 
+bool injected_scratch_failure() {
+    static const long long at = [] {
+        const char* v = std::getenv("ASG_FAIL_SCRATCH_AT");
+        return v ? std::atoll(v) : -1LL;
+    }();
+    static std::atomic<long long> count{0};
+    return at > 0 && count.fetch_add(1) + 1 == at;
+}
+
 int DevBuf::alloc(std::size_t bytes, bool zero) {
     release();
     if (bytes == 0) return ASG_OK;

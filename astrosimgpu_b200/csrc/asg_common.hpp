@@ -39,6 +39,9 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 // the (n+1)-th device allocation of the process fails with out-of-memory.
 // Lets the host error paths be exercised without exhausting a shared GPU.
 bool injected_alloc_failure();
+// ASG_FAIL_SCRATCH_AT=n: the n-th allocation of an admission's device memory
+// (scratch or arena) fails, that one alone.
+bool injected_scratch_failure();
 
 // Host-side NVTX range over a scope, named after the reference's phase
 // table where one applies (Network::run's PhaseProfile, network.hpp:32-45:

@@ -79,9 +79,11 @@ AstroK make_astro_k(const asg_astro_params& a, double h, int substeps) {
 // A failed allocation reports ASG_ERR_OOM (a server then waits for memory to
 // free up).
 int need(AsyncBuf& buf, std::size_t bytes, const Scratch& sc) {
-    const cudaError_t e = buf.alloc(bytes, sc);
+    const cudaError_t e =
+        injected_scratch_failure() ? cudaErrorMemoryAllocation : buf.alloc(bytes, sc);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
+        if (sc.no_room) *sc.no_room = true;
         return fail(ASG_ERR_OOM, "admission: %zu device bytes unavailable", bytes);
     }
     return e == cudaSuccess ? ASG_OK : cuda_fail(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
@@ -472,10 +474,10 @@ int check_csr(const char* name, const asg_csr& c, std::uint32_t n_src) {
 // Targets in range: a small set on the host, a larger one uploaded (it is
 // needed there next) and scanned on the device; `t.bad` is read once the
 // stream has been synchronised.
-int scan_targets(const asg_csr& c, std::uint32_t n_src, std::uint32_t n_tgt, const Scratch& sc,
-                 AsyncBuf& flag, SetTargets& t) {
+int scan_targets(const asg_csr& c, std::uint32_t n_src, std::uint32_t n_tgt, bool on_device,
+                 const Scratch& sc, AsyncBuf& flag, SetTargets& t) {
     const std::uint32_t m = n_src ? c.row_start[n_src] : 0;
-    const bool here = m < kDeviceEdges || m >= (1u << 31);
+    const bool here = !on_device || m < kDeviceEdges || m >= (1u << 31);
     if (here || need(flag, 4, sc) != ASG_OK ||
         need(t.tg, static_cast<std::size_t>(m) * 4, sc) != ASG_OK) {
         clear_error();  // no room for the scan there
@@ -716,7 +718,16 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
                     std::int64_t end, bool keep_spikes, bool check_budget,
                     std::unique_ptr<Instance>* out) {
     NvtxRange nvtx("admission: prepare instance");
-    const int st = prepare_instance(d, rec, first, end, keep_spikes, check_budget, out);
+    bool no_room = false;
+    int st = prepare_instance(d, rec, first, end, keep_spikes, check_budget, true, &no_room, out);
+    if (st == ASG_ERR_OOM && no_room) {
+        // The device holds every set's targets and the SIC lists beside the ring
+        // being numbered: once more with one set at a time, from the host's tables.
+        clear_error();
+        cudaStreamSynchronize(upload);
+        cudaMemPoolTrimTo(pool, 0);
+        st = prepare_instance(d, rec, first, end, keep_spikes, check_budget, false, nullptr, out);
+    }
     if (!cfg.keep_memory) {  // the scratch goes back (its frees are on the stream)
         cudaStreamSynchronize(upload);
         cudaMemPoolTrimTo(pool, 0);
@@ -726,7 +737,8 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
 
 int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* rec,
                              std::int64_t first, std::int64_t end, bool keep_spikes,
-                             bool check_budget, std::unique_ptr<Instance>* out) {
+                             bool check_budget, bool on_device, bool* no_room,
+                             std::unique_ptr<Instance>* out) {
     // Touches no state the chunks in flight use: the tables are prepared and
     // uploaded on the upload stream into a new arena, so a serving loop can
     // run this on another thread while the engine's stream keeps stepping.
@@ -745,7 +757,7 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
     ASG_TRY(check_csr("inh_primary", d.inh_primary, NI));
     ASG_TRY(check_csr("neuron_astro", d.neuron_astro, NE));
     ASG_TRY(check_csr("astro_neuron", d.astro_neuron, NA));
-    const Scratch sc{upload, pool};
+    const Scratch sc{upload, pool, no_room};
     SetTargets on_exc, on_inh, on_n2a, on_a2n;
     {
         struct {
@@ -760,7 +772,8 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
         AsyncBuf flags[4];
         int st = ASG_OK;
         for (int k = 0; k < 4 && st == ASG_OK; ++k)
-            st = scan_targets(*sets[k].c, sets[k].n_src, sets[k].n_tgt, sc, flags[k], *sets[k].t);
+            st = scan_targets(*sets[k].c, sets[k].n_src, sets[k].n_tgt, on_device, sc, flags[k],
+                              *sets[k].t);
         ASG_CUDA(cudaStreamSynchronize(upload));  // the flags, also before an early return
         ASG_TRY(st);
         for (const auto& k : sets)
@@ -982,6 +995,8 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
         if (st == ASG_ERR_OOM) clear_error();  // no room for the sort: on the host
         sic_on_device = st == ASG_OK;
     }
+    on_a2n.tg.release();
+    sic_dev.deg.release();
     if (!sic_on_device)
         sic = make_sic(NA, rs_of(d.astro_neuron), d.astro_neuron.target, N,
                        static_cast<std::uint32_t>(D.sic_parts), D.sic_npad);
@@ -1089,7 +1104,7 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
                     static_cast<unsigned long long>(cfg.mem_budget));
     if (injected_alloc_failure())
         return fail(ASG_ERR_OOM, "device allocation of %zu bytes refused (injected failure)", total);
-    const Scratch keep{upload, cfg.keep_memory ? pool : nullptr};
+    const Scratch keep{upload, cfg.keep_memory ? pool : nullptr, no_room};
     ASG_TRY(need(I.arena, total, keep));
     I.arena_bytes = total;
     {

@@ -38,6 +38,7 @@ struct SpikeRec {
 struct Scratch {
     cudaStream_t stream;
     cudaMemPool_t pool;
+    bool* no_room = nullptr;  // set when an allocation failed for lack of memory
 };
 
 // Device memory from there.  Freeing pool memory does not wait for the device
@@ -57,10 +58,12 @@ struct AsyncBuf {
     void* get() const { return p; }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
-    ~AsyncBuf() {
+    void release() {
         if (p && from.pool) cudaFreeAsync(p, from.stream);
         if (p && !from.pool) cudaFree(p);
+        p = nullptr;
     }
+    ~AsyncBuf() { release(); }
 };
 
 // Mapped host buffers (spike logs, record rows) that leaving instances give
@@ -263,8 +266,8 @@ private:
     cudaStream_t upload = nullptr;  // table uploads of add(), beside the chunks in flight
     cudaMemPool_t pool = nullptr;  // admission scratch (and a server's arenas)
     int prepare_instance(const asg_network_desc& d, const asg_record_opts* rec, std::int64_t first,
-                         std::int64_t end, bool keep_spikes, bool check_budget,
-                         std::unique_ptr<Instance>* out);
+                         std::int64_t end, bool keep_spikes, bool check_budget, bool on_device,
+                         bool* no_room, std::unique_ptr<Instance>* out);
     std::shared_ptr<HostPool> host_pool = std::make_shared<HostPool>();
     std::vector<Work> side_work;
     DevBuf d_side_work;
