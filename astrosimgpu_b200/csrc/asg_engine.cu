@@ -1266,6 +1266,78 @@ int Engine::hold_span_buffers() {
     return ASG_OK;
 }
 
+// The work table of launches of one step or of several.  Push and SIC blocks
+// first (longest dependent chains), then neurons, then astrocytes; in the wide
+// form of several-step launches the longest items first -- neurons, then
+// astrocytes, which balances the blocks' last items -- and a quarter of the push
+// blocks, last: their pushes have the whole launch's time (10^6 neurons 81.5 ->
+// 80.4 us per step, 50,000 5.90 -> 5.63, the 64-instance sweep 7.50 -> 7.37).  A
+// PUSH item's `first` is its index among the instance's push blocks.
+//
+// Step kernel form: a large step is throughput-bound and the wide form runs
+// it faster; a smaller one is bound by its dependent round trips, which the
+// latency form keeps fewest.  Launches of one step: the line lies at two
+// waves of the latency form (4 blocks of 128 threads per SM).  Launches of
+// several: a little above one wave of it (3 per SM); per step, latency and
+// wide form: 25,000 neurons (490 items) 3.17 and 3.59 us, 30,000 (588) 4.22
+// and 3.60, 60,000 7.47 and 6.01.
+void Engine::fill_table(bool several) {
+    Table& T = tables[several];
+    const std::size_t n = insts.size();
+    const int B = cfg.block;
+    const auto fill = [&](bool wide) {
+        T.work.clear();
+        T.push_blocks.assign(n, 0);
+        T.push_helpers.assign(n, 0);
+        if (several && span == 1) return;
+        for (int at = 0; at < 4; ++at) {
+            const int role = several && wide ? (at + 2) % 4 : at;
+            for (std::size_t s = 0; s < n; ++s) {
+                const InstDev& D = insts[s]->dev;
+                const std::uint16_t r = role == 0   ? kRolePush
+                                        : role == 1 ? kRoleSic
+                                        : role == 2 ? kRoleNeuron
+                                                    : kRoleAstro;
+                if (r == kRoleSic && (D.fused_sic || (D.sic_inline && several) ||
+                                      (D.sic_side && cfg.use_graphs != 2)))
+                    continue;
+                if (r == kRolePush) {
+                    if (!D.deferred_push) continue;
+                    const int all = insts[s]->step_push_blocks;
+                    T.push_blocks[s] = several && wide ? (all + 3) / 4 : all;
+                    for (int pb = 0; pb < T.push_blocks[s]; ++pb)
+                        T.work.push_back(Work{static_cast<std::uint32_t>(s), r, kNoHelper,
+                                              static_cast<std::uint32_t>(pb), 0});
+                    continue;
+                }
+                const std::uint32_t cells = r == kRoleAstro ? D.NA
+                                            : r == kRoleSic
+                                                ? static_cast<std::uint32_t>(D.sic_parts) * D.sic_npad
+                                                : D.N;
+                for (std::uint32_t f = 0; f < cells; f += B) {
+                    const std::uint16_t h =
+                        D.deferred_push && T.push_helpers[s] < kNoHelper
+                            ? static_cast<std::uint16_t>(T.push_helpers[s]++)
+                            : kNoHelper;
+                    T.work.push_back(Work{static_cast<std::uint32_t>(s), r, h, f,
+                                          std::min<std::uint32_t>(B, cells - f)});
+                }
+            }
+        }
+    };
+    fill(false);
+    const std::size_t line = static_cast<std::size_t>(several ? 7 * sms / 2 : 8 * sms);
+    T.wide = B == 128 && (cfg.occupancy == 2 || (cfg.occupancy == 0 && T.work.size() > line));
+    if (T.wide && several) fill(true);
+    // The large forms run as one wave of resident blocks, each taking several
+    // work items (no per-item block launch or descriptor staging after its
+    // first).
+    T.grid = T.wide && cfg.item_loop
+                 ? sms * step_blocks_per_sm(several ? StepForm::kSpanWide : StepForm::kWide,
+                                            cfg.astro_fp32)
+                 : 0;
+}
+
 int Engine::rebuild() {
     ASG_TRY(finish_pending());
     ASG_CUDA(cudaStreamSynchronize(stream));
@@ -1305,64 +1377,7 @@ int Engine::rebuild() {
         D.fany_ahead = p->fac_in_span ? kMaxSpan : 1;
         if (span == 1) p->span.reset();
     }
-    // The work table.  Push and SIC blocks first (longest dependent chains),
-    // then neurons, then astrocytes; in the wide form of several-step launches
-    // the longest items first -- neurons, then astrocytes, which balances the
-    // blocks' last items -- and a quarter of the push blocks, last: their
-    // pushes have the whole launch's time (10^6 neurons 81.5 -> 80.4 us per step,
-    // 50,000 5.90 -> 5.63, the 64-instance sweep 7.50 -> 7.37).  A PUSH item's
-    // `first` is its index among the instance's push blocks.
-    std::vector<std::uint32_t> helpers;
-    auto fill_work = [&](bool span_wide) {
-        work.clear();
-        helpers.assign(insts.size(), 0);
-        for (int at = 0; at < 4; ++at) {
-            const int role = span_wide ? (at + 2) % 4 : at;
-            for (std::size_t s = 0; s < insts.size(); ++s) {
-                InstDev& D = insts[s]->dev;
-                const std::uint16_t r = role == 0   ? kRolePush
-                                        : role == 1 ? kRoleSic
-                                        : role == 2 ? kRoleNeuron
-                                                    : kRoleAstro;
-                if (r == kRoleSic && (D.fused_sic || D.sic_inline || (D.sic_side && cfg.use_graphs != 2)))
-                    continue;
-                if (r == kRolePush) {
-                    if (!D.deferred_push) continue;
-                    D.push_blocks = span_wide ? (insts[s]->step_push_blocks + 3) / 4
-                                              : insts[s]->step_push_blocks;
-                    for (int pb = 0; pb < D.push_blocks; ++pb)
-                        work.push_back(Work{static_cast<std::uint32_t>(s), r, kNoHelper,
-                                            static_cast<std::uint32_t>(pb), 0});
-                    continue;
-                }
-                const std::uint32_t n = r == kRoleAstro ? D.NA
-                                        : r == kRoleSic
-                                            ? static_cast<std::uint32_t>(D.sic_parts) * D.sic_npad
-                                            : D.N;
-                for (std::uint32_t f = 0; f < n; f += B) {
-                    const std::uint16_t h = D.deferred_push && helpers[s] < kNoHelper
-                                                ? static_cast<std::uint16_t>(helpers[s]++)
-                                                : kNoHelper;
-                    work.push_back(Work{static_cast<std::uint32_t>(s), r, h, f,
-                                        std::min<std::uint32_t>(B, n - f)});
-                }
-            }
-        }
-    };
-    fill_work(false);
-    // Step kernel form: a large step is throughput-bound and the wide form runs
-    // it faster; a smaller one is bound by its dependent round trips, which the
-    // latency form keeps fewest.  Launches of one step: the line lies at two
-    // waves of the latency form (4 blocks of 128 threads per SM).  Launches of
-    // several: a little above one wave of it (3 per SM); per step, latency and
-    // wide form: 25,000 neurons (490 items) 3.17 and 3.59 us, 30,000 (588) 4.22
-    // and 3.60, 60,000 7.47 and 6.01.
-    const std::size_t line = span > 1 ? static_cast<std::size_t>(7 * sms / 2)
-                                      : static_cast<std::size_t>(8 * sms);
-    wide = cfg.block == 128 && (cfg.occupancy == 2 || (cfg.occupancy == 0 && work.size() > line));
-    if (wide && span > 1) fill_work(true);
-    for (std::size_t s = 0; s < insts.size(); ++s)
-        insts[s]->dev.push_helpers = static_cast<std::int32_t>(helpers[s]);
+    for (bool several : {false, true}) fill_table(several);
     // Side-stream SIC batches (graph and plain launches; the persistent
     // kernel computes the single-part sums in its SIC role instead).
     side_work.clear();
@@ -1380,7 +1395,9 @@ int Engine::rebuild() {
                                          std::min<std::uint32_t>(B, D.N - f)});
         }
     }
-    if (insts.size() > cap_insts || work.size() * sizeof(Work) > d_work.bytes()) {
+    tables[1].at = tables[0].work.size();
+    const std::size_t items = tables[0].work.size() + tables[1].work.size();
+    if (insts.size() > cap_insts || items * sizeof(Work) > d_work.bytes()) {
         const std::size_t cap = std::max<std::size_t>(insts.size(), 1);
         if (cap > cap_insts) {
             const std::size_t c2 = std::max(cap, cap_insts * 2);
@@ -1397,12 +1414,13 @@ int Engine::rebuild() {
             }
             cap_insts = c2;
         }
-        if (work.size() * sizeof(Work) > d_work.bytes())
-            ASG_TRY(d_work.alloc(std::max<std::size_t>(work.size(), 64) * 2 * sizeof(Work)));
+        if (items * sizeof(Work) > d_work.bytes())
+            ASG_TRY(d_work.alloc(std::max<std::size_t>(items, 64) * 2 * sizeof(Work)));
     }
-    if (!work.empty())
-        ASG_CUDA(cudaMemcpyAsync(d_work.get(), work.data(), work.size() * sizeof(Work),
-                                 cudaMemcpyHostToDevice, stream));
+    for (const Table& T : tables)
+        if (!T.work.empty())
+            ASG_CUDA(cudaMemcpyAsync(d_work.as<Work>() + T.at, T.work.data(),
+                                     T.work.size() * sizeof(Work), cudaMemcpyHostToDevice, stream));
     if (side_work.size() * sizeof(Work) > d_side_work.bytes())
         ASG_TRY(d_side_work.alloc(side_work.size() * 2 * sizeof(Work)));
     if (!side_work.empty())
@@ -1411,21 +1429,14 @@ int Engine::rebuild() {
     ASG_CUDA(cudaMemsetAsync(d_stats.get(), 0, cap_insts * kStatWords * sizeof(unsigned long long),
                              stream));
     ASG_CUDA(cudaStreamSynchronize(stream));
-    // The large forms run as one wave of resident blocks, each taking several
-    // work items (no per-item block launch or descriptor staging after its
-    // first).
-    wide_grid = 0;
-    if (wide && cfg.item_loop)
-        wide_grid = sms * step_blocks_per_sm(span > 1 ? StepForm::kSpanWide : StepForm::kWide,
-                                             cfg.astro_fp32);
     persistent_grid = 0;
-    if (cfg.use_graphs == 2 && !work.empty()) {
+    if (cfg.use_graphs == 2 && !tables[0].work.empty()) {
         const int cap = persistent_blocks(B);
         if (cap <= 0) return fail(ASG_ERR_CUDA, "persistent kernel: no co-resident blocks");
-        persistent_grid = std::min<int>(cap, static_cast<int>(work.size()));
+        persistent_grid = std::min<int>(cap, static_cast<int>(tables[0].work.size()));
     }
     dirty = false;
-    if (graph_mode() && !work.empty()) ASG_TRY(capture_graph(cfg.chunk_steps));
+    if (graph_mode() && !tables[0].work.empty()) ASG_TRY(capture_graph(cfg.chunk_steps));
     return ASG_OK;
 }
 
@@ -1478,7 +1489,7 @@ int Engine::capture_graph(int steps) {
 // pushes from it, before that.
 std::vector<Span> Engine::plan(int steps) const {
     std::vector<Span> v;
-    if (span == 1 || steps < span + 2) {
+    if (!several_steps(steps)) {
         for (int k = 0; k < steps; ++k) v.push_back(Span{k, 1, k - 1, 0, 3, 3, -1, 0});
         return v;
     }
@@ -1510,8 +1521,10 @@ cudaError_t Engine::issue_steps(int steps) {
                    "update neurons, spike delivery, SIC gather+deliver");
     const bool side_on = !side_work.empty();
     const int G = kSicBatchSteps;
-    const StepForm form = span > 1 ? (wide ? StepForm::kSpanWide : StepForm::kSpan)
-                                   : (wide ? StepForm::kWide : StepForm::kLatency);
+    const bool several = several_steps(steps);
+    const Table& T = tables[several];
+    const StepForm form = several ? (T.wide ? StepForm::kSpanWide : StepForm::kSpan)
+                                  : (T.wide ? StepForm::kWide : StepForm::kLatency);
     cudaError_t e = cudaSuccess;
     if (side_on) {
         e = cudaEventRecord(ev_side_fork, stream);
@@ -1536,9 +1549,9 @@ cudaError_t Engine::issue_steps(int steps) {
             if (k >= side_lead && (k - side_lead) % G == 0)
                 e = cudaStreamWaitEvent(stream, ev_side_done[((k - side_lead) / G) % kSideEvents], 0);
         if (e == cudaSuccess)
-            e = launch_step(d_insts.as<InstDev>(), d_work.as<Work>(), static_cast<int>(work.size()),
-                            cfg.block, sp, cfg.pdl && sp.k > 0, form, wide ? wide_grid : 0,
-                            cfg.astro_fp32, stream);
+            e = launch_step(d_insts.as<InstDev>(), d_work.as<Work>() + T.at,
+                            static_cast<int>(T.work.size()), cfg.block, sp, cfg.pdl && sp.k > 0,
+                            form, T.grid, cfg.astro_fp32, stream);
     }
     if (side_on && e == cudaSuccess) {
         e = cudaEventRecord(ev_side_join, side);
@@ -1610,6 +1623,8 @@ cudaError_t Engine::prime_side() {
 }
 
 int Engine::launch_chunk(int parity, int steps) {
+    const bool several = several_steps(steps);
+    const Table& T = tables[several];
     // Stage the descriptors: step window of this chunk, output pointers.
     InstDev* hi = h_insts[parity];
     for (std::size_t s = 0; s < insts.size(); ++s) {
@@ -1617,6 +1632,8 @@ int Engine::launch_chunk(int parity, int steps) {
         InstDev D = I.dev;
         D.step0 = I.step;
         D.end_step = std::min<std::int64_t>(I.end, I.step + steps);
+        D.push_blocks = T.push_blocks[s];
+        D.push_helpers = T.push_helpers[s];
         unsigned long long* st = d_stats.as<unsigned long long>() + s * kStatWords;
         D.spike_log_n = st;
         D.counters = st + 1;
@@ -1642,7 +1659,7 @@ int Engine::launch_chunk(int parity, int steps) {
     if (persistent_grid > 0) {
         ASG_CUDA(cudaMemsetAsync(d_barrier.get(), 0, sizeof(GridBarrier), stream));
         ASG_CUDA(launch_chunk_persistent(d_insts.as<InstDev>(), d_work.as<Work>(),
-                                         static_cast<int>(work.size()), cfg.block,
+                                         static_cast<int>(T.work.size()), cfg.block,
                                          persistent_grid, steps, d_barrier.as<GridBarrier>(),
                                          cfg.astro_fp32, stream));
         ASG_CUDA(cudaMemcpyAsync(h_barrier_err[parity], &d_barrier.as<GridBarrier>()->error,
@@ -1746,7 +1763,7 @@ int Engine::run_chunk(std::int64_t max_steps) {
     std::int64_t steps = 0;
     for (auto& p : insts) steps = std::max<std::int64_t>(steps, p->end - p->step);
     steps = std::min<std::int64_t>({steps, max_steps, cfg.chunk_steps});
-    if (steps <= 0 || work.empty()) return ASG_OK;
+    if (steps <= 0 || tables[0].work.empty()) return ASG_OK;
     // Two chunks in flight: the host collects one while the next runs.
     const int p = next_parity;
     ASG_TRY(collect(p));
@@ -1784,7 +1801,7 @@ int Engine::run(std::int64_t n_steps) {
         return (l + c - 1) / c;
     };
     int st = ASG_OK;
-    if (graph_mode() && !work.empty()) {
+    if (graph_mode() && !tables[0].work.empty()) {
         for (std::int64_t l = left(), prev = 0; l > 0 && st == ASG_OK; l -= prev) {
             const std::int64_t a = next_chunk(l);
             if (a != prev) st = capture_graph(static_cast<int>(a));

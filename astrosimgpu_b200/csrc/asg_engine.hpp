@@ -228,6 +228,13 @@ public:
 
 private:
     int rebuild();          // work table + graph after the instance set changed
+    // The launches of a chunk of `steps` steps take several each, or one where a
+    // chunk is too short to begin, go on and end (see plan).  A call of a few
+    // steps runs the single-step kernels as any engine without several steps does:
+    // through the several-step kernels, one step at a time, calls of 1, 5 and 6 steps
+    // took 79 -> 89 us (200,000 neurons), 25.4 -> 26.5 and 23.4 -> 25.0 us per step
+    // (100,000).
+    bool several_steps(int steps) const { return span > 1 && steps >= span + 2; }
     std::vector<Span> plan(int steps) const;  // the launches of a chunk
     cudaError_t issue_steps(int steps);  // step launches + side-stream SIC batches
     int copy_factors(Instance& I, bool to_span);
@@ -248,14 +255,21 @@ private:
     unsigned* h_barrier_err[2] = {nullptr, nullptr};  // pinned copy of its error word
     int persistent_grid = 0;
     std::size_t cap_insts = 0;
-    std::vector<Work> work;
+    // The work of one launch: [0] of one step, [1] of several.
+    struct Table {
+        std::vector<Work> work;
+        std::vector<std::int32_t> push_blocks, push_helpers;  // by instance
+        std::size_t at = 0;  // first item in d_work
+        bool wide = false;   // the high-occupancy form of the kernel
+        int grid = 0;        // its grid: one wave of resident blocks (0: one block per item)
+    };
+    Table tables[2];
+    void fill_table(bool several);
     // Captured chunk graphs by length, most recently used first: the
     // chunk_steps graph and the lengths run() splits its calls into.
     static constexpr std::size_t kMaxGraphs = 4;
     std::vector<std::pair<int, cudaGraphExec_t>> graphs;
     bool graph_mode() const { return cfg.use_graphs == 0 || cfg.use_graphs == 1; }
-    bool wide = false;  // launches use the high-occupancy form of the step kernel
-    int wide_grid = 0;  // its grid: one wave of resident blocks (0: one block per item)
     cudaGraphExec_t find_graph(int steps);
     int capture_graph(int steps);
     void drop_graphs();

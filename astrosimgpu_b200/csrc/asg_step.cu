@@ -94,7 +94,7 @@ __device__ void make_step_info(const InstDev& I, std::int64_t step, std::int64_t
     if (lane == 11) { d = I.pi.steps_per_noise; }
     if (lane == 12) { d = I.a_steps_per_noise; }
     if (lane >= 13 && lane < 13 + P) { n = step + P - (lane - 13) - I.d_a2n; d = I.sic_interval; }
-    if (lane >= 13 + P && lane < 13 + 2 * P) { n = step + P - (lane - 13 - P) - I.d_a2n; }
+    if (lane >= 13 + P && lane < 13 + 2 * P) { n = step + P - (lane - 13 - P) - I.d_a2n; d = I.fac_slots; }
     // (eight parts leave no lane, but then the factors are the arena's)
     if (lane == 28 && P < 8) { d = I.fac_slots; }
     if (lane == 29) { d = I.fany_slots; }
@@ -1211,7 +1211,7 @@ __device__ void push_role(const InstDev& I, const StepInfo& S, const Span& sp, c
     if (kPdl) grid_dep_wait();
     if (wk.first == 0 && threadIdx.x == 0) {
         if (kSpan && sp.clear >= 0) I.span_packed[sp.clear * kHeaderStride] = 0;
-        if ((!kSpan || (sp.src == 3 && sp.dst == 3)) && S.step < I.end_step)
+        if (!kSpan && S.step < I.end_step)
             I.spk_packed[S.ls_next * kHeaderStride] = 0;
         if (kSpan && sp.clear_arena && I.step0 < I.end_step)
             for (int l = 0; l < 3; ++l) I.spk_packed[l * kHeaderStride] = 0;
