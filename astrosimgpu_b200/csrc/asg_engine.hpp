@@ -242,6 +242,10 @@ private:
     int span = 1;  // most steps per launch
     int launch_chunk(int parity, int steps);
     int collect(int parity);
+    void order_spikes(const unsigned long long* log, std::size_t n, std::int64_t first,
+                      std::int64_t last, std::vector<SpikeRec>& out);
+    std::vector<std::size_t> step_end;  // its scratch
+    std::vector<std::uint32_t> by_step;
     int finish_pending();
 
     DevBuf d_insts, d_work;
