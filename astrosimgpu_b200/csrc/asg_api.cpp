@@ -225,6 +225,7 @@ int asg_create(const asg_network_desc* desc, const asg_record_opts* rec,
     h->eng = std::make_unique<Engine>(cfg);
     ASG_TRY(h->eng->init());
     ASG_TRY(h->eng->add(*desc, rec, 0, INT64_MAX, true, &h->id));
+    h->eng->release_scratch();
     *out = reinterpret_cast<asg_network*>(h.release());
     return ASG_OK;
 }
@@ -367,6 +368,7 @@ int asg_batch_create(int32_t n, const asg_network_desc* const* descs, const asg_
         if (st != ASG_OK) return st;
         h->ids.push_back(id);
     }
+    h->eng->release_scratch();
     *out = reinterpret_cast<asg_batch*>(h.release());
     return ASG_OK;
 }

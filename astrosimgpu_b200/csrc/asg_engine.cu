@@ -724,15 +724,15 @@ int Engine::prepare(const asg_network_desc& d, const asg_record_opts* rec, std::
         // The device holds every set's targets and the SIC lists beside the ring
         // being numbered: once more with one set at a time, from the host's tables.
         clear_error();
-        cudaStreamSynchronize(upload);
-        cudaMemPoolTrimTo(pool, 0);
+        release_scratch();
         st = prepare_instance(d, rec, first, end, keep_spikes, check_budget, false, nullptr, out);
     }
-    if (!cfg.keep_memory) {  // the scratch goes back (its frees are on the stream)
-        cudaStreamSynchronize(upload);
-        cudaMemPoolTrimTo(pool, 0);
-    }
     return st;
+}
+
+void Engine::release_scratch() {
+    cudaStreamSynchronize(upload);  // the frees are on the stream
+    cudaMemPoolTrimTo(pool, 0);
 }
 
 int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* rec,

@@ -33,7 +33,7 @@ struct SpikeRec {
 // device and, beside running chunks, took from 0.4 to tens of ms each.)  A
 // server's pool also holds the arenas and keeps up to 2 GB beside them, within
 // the memory budget, between requests (Engine::claim); other engines trim it
-// after each admission and take their arenas, which stay, from cudaMalloc
+// after their last admission and take their arenas, which stay, from cudaMalloc
 // (pool = nullptr).
 struct Scratch {
     cudaStream_t stream;
@@ -171,6 +171,9 @@ public:
     int prepare(const asg_network_desc& d, const asg_record_opts* rec, std::int64_t first,
                 std::int64_t end, bool keep_spikes, bool check_budget,
                 std::unique_ptr<Instance>* out);
+    // Gives the memory that admissions worked in back to the device (an engine
+    // whose instances stay: after the last of them).
+    void release_scratch();
     // Joins a prepared instance at this chunk boundary (same thread as run).
     int commit(std::unique_ptr<Instance> inst, int* id);
     int remove(int id);
