@@ -984,7 +984,9 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
         const int ref = NE == 0 ? D.pi.ref_steps
                         : NI == 0 ? D.pe.ref_steps
                                   : std::min(D.pe.ref_steps, D.pi.ref_steps);
-        L = span_that_fits(L, N, edges, d.substeps, ref);
+        // 28 bits in the wide form, which a network of more than ~66,000 cells
+        // runs unless the caller asks for the latency form's 24
+        L = span_that_fits(L, N, edges, d.substeps, ref, cfg.occupancy == 1 ? 24 : 28);
         I.span_max = std::max(1, L);
     }
     SicHost sic;

@@ -148,7 +148,8 @@ struct InstDev {
     InRing ring_ex, ring_in, ring_as;
     // Deferred push (both spike delays >= 2 steps): each spike of step s
     // reserves a contiguous range of that step's flat edge space (one 64-bit
-    // atomic: list index in the high bits, edge offset in the low 40) and is
+    // atomic: list index in the high bits, edge offset in the low 40 -- 36 in
+    // the wide form's launches of several steps) and is
     // pushed in step s+1 by the PUSH blocks, whose threads stride over the
     // flat space -- every edge of every spike gets one thread, whatever the
     // spike count.  Three list slots rotate: append (s), push (s-1), reset (s+1).

@@ -162,6 +162,16 @@ __device__ __forceinline__ int span_count(const InstDev& I, std::int64_t first, 
     return left < cnt ? static_cast<int>(left) : cnt;
 }
 
+// Low bits of a spike list's header word that hold the edge total, the record
+// count above them: 40 in the arena's lists (a step lists a cell once, and fewer
+// than 2^24 cells), 36 in those of the wide form's launches of several steps.  The
+// latency form keeps 40 there too (span_that_fits): a choice at run time cost it
+// 0.5 % (5,000 neurons 2.495 -> 2.508 us per step).
+template <bool kWide, bool kSpan>
+__device__ __forceinline__ int edge_bits(int list) {
+    return kWide && kSpan && list != 3 ? 36 : 40;
+}
+
 // A spike list: its header word and its records.
 struct SpikeList {
     unsigned long long* packed;
@@ -954,10 +964,11 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
                     if (I.deferred_push) {
                         const SpikeList L = spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i);
                         const unsigned long long old = atomicAdd(
-                            L.packed, (1ull << 40) | static_cast<unsigned long long>(len0 + len1));
-                        const std::size_t o = old >> 40;
+                            L.packed, (1ull << edge_bits<kWide, kSpan>(sp.dst)) |
+                                          static_cast<unsigned long long>(len0 + len1));
+                        const std::size_t o = old >> edge_bits<kWide, kSpan>(sp.dst);
                         *reinterpret_cast<uint4*>(L.meta + 4 * o) =
-                            make_uint4(r1, static_cast<std::uint32_t>(old & 0xFFFFFFFFFFull), r0,
+                            make_uint4(r1, static_cast<std::uint32_t>(old), r0,
                                        kSpan ? len0 | static_cast<std::uint32_t>(j) << 28 : len0);
                         *reinterpret_cast<double2*>(L.val + 2 * o) = make_double2(v0, v1);
                     }
@@ -1004,7 +1015,8 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
                 if (lane == static_cast<unsigned>(leader)) {
                     if (I.deferred_push)
                         base_spk = atomicAdd(spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i).packed,
-                                             (static_cast<unsigned long long>(nspk) << 40) | total);
+                                             (static_cast<unsigned long long>(nspk)
+                                              << edge_bits<kWide, kSpan>(sp.dst)) | total);
                     if (logging) base_log = atomicAdd(I.spike_log_n, static_cast<unsigned long long>(nspk));
                     atomicAdd(I.counters + 0, total);
                     atomicAdd(I.counters + 2, static_cast<unsigned long long>(nspk));
@@ -1014,8 +1026,8 @@ __device__ void neuron_role(const InstDev& I, const StepInfo* __restrict__ S, co
                 if (spiked) {
                     if (I.deferred_push) {
                         const SpikeList L = spike_list<kSpan>(I, sp.dst, S[0].ls, sp.i);
-                        const std::size_t o = (base_spk >> 40) + rank;
-                        const unsigned long long eoff = (base_spk & 0xFFFFFFFFFFull) + (incl - edges);
+                        const std::size_t o = (base_spk >> edge_bits<kWide, kSpan>(sp.dst)) + rank;
+                        const unsigned long long eoff = base_spk + (incl - edges);  // low 32 bits
                         *reinterpret_cast<uint4*>(L.meta + 4 * o) =
                             make_uint4(r1, static_cast<std::uint32_t>(eoff), r0,
                                        kSpan ? len0 | static_cast<std::uint32_t>(j) << 28 : len0);
@@ -1083,13 +1095,13 @@ constexpr int kPushBatch = 256;
 // 0.16 us slower per paper-sparse step there.
 template <bool kDealt, bool kSpan>
 __device__ void push_spikes(const InstDev& I, const StepInfo& S, const SpikeList& L,
-                            unsigned long long packed, std::uint32_t rank,
+                            unsigned long long packed, int bits, std::uint32_t rank,
                             std::uint32_t nranks) {
     __shared__ std::uint32_t s_off[kPushBatch + 1], s_r0[kPushBatch], s_len0[kPushBatch],
         s_r1[kPushBatch], s_slot[kSpan ? kPushBatch : 1];
     __shared__ double s_v[2 * kPushBatch];
-    const std::uint32_t n = static_cast<std::uint32_t>(packed >> 40);
-    const std::uint32_t total = static_cast<std::uint32_t>(packed & 0xFFFFFFFFFFull);
+    const std::uint32_t n = static_cast<std::uint32_t>(packed >> bits);
+    const std::uint32_t total = static_cast<std::uint32_t>(packed);
     if (n == 0) return;  // block-uniform
     const std::uint32_t nbatch = (n + kPushBatch - 1) / kPushBatch;
     const std::uint32_t slots = static_cast<std::uint32_t>(I.slots);
@@ -1189,8 +1201,8 @@ __device__ void push_spikes(const InstDev& I, const StepInfo& S, const SpikeList
 // A burst: more than kBurstEdgesPerThread spike edges per push thread.
 constexpr std::uint32_t kBurstEdgesPerThread = 4;
 
-__device__ __forceinline__ bool push_burst(const InstDev& I, unsigned long long packed) {
-    return (packed & 0xFFFFFFFFFFull) >
+__device__ __forceinline__ bool push_burst(const InstDev& I, unsigned long long packed, int bits) {
+    return (packed & ((1ull << bits) - 1ull)) >
            static_cast<unsigned long long>(kBurstEdgesPerThread) * blockDim.x * I.push_blocks;
 }
 
@@ -1219,17 +1231,19 @@ __device__ void push_role(const InstDev& I, const StepInfo& S, const Span& sp, c
     if (!push_pending<kSpan>(I, S, sp)) return;
     const SpikeList L = spike_list<kSpan>(I, sp.src, S.ls_prev, sp.i - 1);
     const unsigned long long packed = __ldcg(L.packed);
+    const int bits = edge_bits<kWide, kSpan>(sp.src);
     const std::uint32_t nranks = static_cast<std::uint32_t>(I.push_blocks) +
-                                 (push_burst(I, packed) ? I.push_helpers : 0u);
-    push_spikes<kWide, kSpan>(I, S, L, packed, wk.first, nranks);
+                                 (push_burst(I, packed, bits) ? I.push_helpers : 0u);
+    push_spikes<kWide, kSpan>(I, S, L, packed, bits, wk.first, nranks);
 }
 
 // A non-push block's share of a burst push (its rank among the helpers).
 template <bool kWide, bool kSpan>
 __device__ __noinline__ void help_push_spikes(const InstDev& I, const StepInfo& S,
                                               const SpikeList& L, unsigned long long packed,
-                                              std::uint32_t helper) {
-    push_spikes<kWide, kSpan>(I, S, L, packed, static_cast<std::uint32_t>(I.push_blocks) + helper,
+                                              int bits, std::uint32_t helper) {
+    push_spikes<kWide, kSpan>(I, S, L, packed, bits,
+                       static_cast<std::uint32_t>(I.push_blocks) + helper,
                        static_cast<std::uint32_t>(I.push_blocks + I.push_helpers));
 }
 
@@ -1245,8 +1259,9 @@ __device__ __forceinline__ int help_push(const InstDev& I, const StepInfo& S, co
         return burst;
     const SpikeList L = spike_list<kSpan>(I, sp.src, S.ls_prev, sp.i - 1);
     const unsigned long long packed = __ldcg(L.packed);
-    if (!push_burst(I, packed)) return 0;
-    help_push_spikes<kWide, kSpan>(I, S, L, packed, wk.helper);
+    const int bits = edge_bits<kWide, kSpan>(sp.src);
+    if (!push_burst(I, packed, bits)) return 0;
+    help_push_spikes<kWide, kSpan>(I, S, L, packed, bits, wk.helper);
     return 1;
 }
 

@@ -1,5 +1,5 @@
 """A launch of several steps lists a cell once per step it spikes in; the list
-counts records in 24 bits and edges in 32.  span_that_fits
+counts records in 28 bits (24 in the latency form) and edges in 32.  span_that_fits
 (astrosimgpu_b200/csrc/asg_span.hpp) shortens the launch so that both hold
 for a network whose every cell fires as often as its refractory time allows,
 whatever the phase: compared with a count over the substeps."""
@@ -12,13 +12,14 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 # want, neurons, edges, substeps, refractory substeps
-CASES = [(5, 3_355_443, 100, 1, 0), (5, 3_355_444, 100, 1, 0), (8, 2_097_151, 100, 1, 0),
-         (8, 2_097_152, 100, 1, 0), (8, (1 << 24) - 1, 100, 1, 7), (8, (1 << 24) - 1, 100, 1, 6),
-         (8, 1 << 24, 100, 1, 20), (5, 10, 845_571_686, 1, 0), (5, 10, 845_571_687, 1, 0),
+SIZES = [(8, (1 << 25) - 1, 100, 1, 0), (8, 1 << 25, 100, 1, 0), (5, 53_687_091, 100, 1, 0),
+         (5, 53_687_092, 100, 1, 0), (8, (1 << 27) - 1, 100, 1, 7), (8, (1 << 27) - 1, 100, 1, 6),
+         (8, 1 << 28, 100, 1, 20), (5, 10, 845_571_686, 1, 0), (5, 10, 845_571_687, 1, 0),
          (8, 1000, (1 << 32) - (1 << 26), 1, 20), (8, 1000, (1 << 32) - (1 << 26) + 1, 1, 20),
          (8, 4_000_000, 400_000_000, 2, 5), (8, 8_000_000, 900_000_000, 1, 3),
-         (8, 6_000_000, 10, 3, 2), (4, 5_000_000, 10, 1, 1), (1, 1 << 24, 1 << 33, 1, 0),
-         (8, 500, 25_000, 1, 20), (5, 1_000_000, 10**8, 1, 20), (8, 0, 0, 1, 0)]
+         (8, 96_000_000, 10, 3, 2), (4, 80_000_000, 10, 1, 1), (1, 1 << 24, 1 << 33, 1, 0),
+         (8, 500, 25_000, 1, 20), (5, 1_000_000, 10**8, 1, 0), (8, 0, 0, 1, 0)]
+CASES = [c + (28,) for c in SIZES] + [(c[0], c[1] >> 4) + c[2:] + (24,) for c in SIZES]
 
 
 @pytest.fixture(scope="module")
@@ -46,13 +47,13 @@ def counted(steps, substeps, ref):
 
 @pytest.mark.parametrize("k", range(len(CASES)))
 def test_spikes_of_a_launch_fit_its_list(limits, k):
-    want, n, e, substeps, ref = CASES[k]
+    want, n, e, substeps, ref, bits = CASES[k]
     span, *spikes = limits[k]
     assert spikes == [counted(L, substeps, ref) for L in range(1, want + 1)]
 
     def fits(L):
         s = counted(L, substeps, ref)
-        return s * n < 1 << 24 and s * e + (1 << 26) <= 1 << 32
+        return s * n < 1 << bits and s * e + (1 << 26) <= 1 << 32
 
     assert span == max([1] + [L for L in range(2, want + 1) if fits(L)])
 
