@@ -544,22 +544,29 @@ std::size_t align256(std::size_t x) { return (x + 255) & ~static_cast<std::size_
 
 Instance::~Instance() {
     for (int p = 0; p < 2; ++p) {
-        if (log_h[p]) host_pool->give(log_h[p], log_bytes);
-        if (rec_h[p]) host_pool->give(rec_h[p], rec_bytes);
+        if (log_h[p]) host_pool->give(log_h[p], log_bytes[p]);
+        if (rec_h[p]) host_pool->give(rec_h[p], rec_bytes[p]);
     }
 }
 
-cudaError_t HostPool::take(std::size_t bytes, void** p) {
+cudaError_t HostPool::take(std::size_t bytes, void** p, std::size_t* got) {
+    bytes = std::max<std::size_t>(bytes, 4096);  // a page at least
     {
         std::lock_guard<std::mutex> g(mu);
-        for (std::size_t i = 0; i < kept.size(); ++i) {
-            if (kept[i].first != bytes) continue;
-            *p = kept[i].second;
-            held -= bytes;
-            kept.erase(kept.begin() + static_cast<std::ptrdiff_t>(i));
+        std::size_t best = kept.size();
+        for (std::size_t i = 0; i < kept.size(); ++i)
+            if (kept[i].first >= bytes && kept[i].first / 2 <= bytes &&
+                (best == kept.size() || kept[i].first < kept[best].first))
+                best = i;
+        if (best < kept.size()) {
+            *p = kept[best].second;
+            *got = kept[best].first;
+            held -= *got;
+            kept.erase(kept.begin() + static_cast<std::ptrdiff_t>(best));
             return cudaSuccess;
         }
     }
+    *got = bytes;
     return cudaHostAlloc(p, bytes, cudaHostAllocMapped);
 }
 
@@ -1149,20 +1156,14 @@ int Engine::prepare_instance(const asg_network_desc& d, const asg_record_opts* r
     I.max_chunk = cfg.chunk_steps;
     const std::size_t rec_doubles =
         static_cast<std::size_t>(I.rec_rows) * (2 * D.rec_astro_max + 2 * D.rec_neuron_max) + 1;
-    // (a server's sizes are rounded up, so that a later request finds them)
     I.host_pool = host_pool;
-    I.log_bytes = static_cast<std::size_t>(I.log_cap) * 8;
-    I.rec_bytes = rec_doubles * 8;
-    if (cfg.keep_memory) {
-        I.log_bytes = HostPool::rounded(I.log_bytes);
-        I.rec_bytes = HostPool::rounded(I.rec_bytes);
-    }
+    const std::size_t log_bytes = static_cast<std::size_t>(I.log_cap) * 8, rec_bytes = rec_doubles * 8;
     for (int p = 0; p < 2; ++p) {
         if (D.rec_spikes) {
-            ASG_CUDA(host_pool->take(I.log_bytes, reinterpret_cast<void**>(&I.log_h[p])));
+            ASG_CUDA(host_pool->take(log_bytes, reinterpret_cast<void**>(&I.log_h[p]), &I.log_bytes[p]));
             ASG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&I.log_d[p]), I.log_h[p], 0));
         }
-        ASG_CUDA(host_pool->take(I.rec_bytes, reinterpret_cast<void**>(&I.rec_h[p])));
+        ASG_CUDA(host_pool->take(rec_bytes, reinterpret_cast<void**>(&I.rec_h[p]), &I.rec_bytes[p]));
         ASG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&I.rec_d[p]), I.rec_h[p], 0));
     }
     D.spike_log_cap = D.rec_spikes ? I.log_cap : 0;
