@@ -106,7 +106,8 @@ struct BatchHandle {
 // Times candidate launch shapes on a snapshot of every instance (device
 // arena + host bookkeeping restored after each trial, so the simulation is
 // not advanced) and keeps the fastest: chunk length x block size x launch
-// mode (CUDA graph of per-step launches or the persistent chunk kernel).
+// mode (CUDA graph of launches -- of several steps with blocks of 128 where the
+// delays allow, else of one -- or the persistent chunk kernel).
 int autotune_engine(Engine& e, int32_t steps, asg_engine_opts* chosen) {
     ASG_TRY(e.flush());
     // Snapshot every instance (device arena + host-side bookkeeping).

@@ -937,12 +937,14 @@ extern "C" int asg_astro_autotune(asg_astro* s, const double* consts, double h_s
 // in place and allocates nothing.  One launch and no scratch: the kernel forms
 // the reciprocal of each cell's tau_IP3 itself.  (A kernel of its own that
 // left the reciprocals in a static array cost a launch, a pass over 16 bytes
-// per cell and the array's address lookup on the host: 1,000,003 cells 42.3 ->
-// 31.0 us per call, input copy included.)
+// per cell and the array's address lookup on the host: 1,000,003 cells 46.8 ->
+// 39.6 us per call, input copy and the wait for it included.)
 
 namespace asg {
 namespace {
-constexpr std::uint32_t kNoAllocMaxCells = 1u << 20;  // the entry point's limit
+// The entry point's limit, once its scratch array's: callers rely on the refusal
+// and its words.
+constexpr std::uint32_t kNoAllocMaxCells = 1u << 20;
 }  // namespace
 }  // namespace asg
 
@@ -957,8 +959,8 @@ extern "C" int asg_astro_update_noalloc(uint32_t n, double* Ca, double* IP3, dou
     if (n == 0) return ASG_OK;
     if (n > asg::kNoAllocMaxCells)
         return asg::fail(ASG_ERR_ARG,
-                         "asg_astro_update_noalloc: %u cells exceed the %u-cell scratch limit; "
-                         "use asg_astro_create/asg_astro_update for larger populations",
+                         "asg_astro_update_noalloc: %u cells exceed the %u of the entry point's limit "
+                         "(the former scratch limit); use asg_astro_create/asg_astro_update for larger populations",
                          n, asg::kNoAllocMaxCells);
     if (Ca == nullptr || IP3 == nullptr || h == nullptr || ip3_input == nullptr ||
         Ca_tot == nullptr || IP3_0 == nullptr || tau_IP3 == nullptr || delta_IP3 == nullptr ||

@@ -228,7 +228,7 @@ struct InstDev {
 // round trip are paid once per launch instead of once per step.  With delays
 // of ten steps (five per launch), per step: 500 neurons 3.32 -> 2.05 us (a step
 // is now its RK4 chain, ~1.1 us, the rest of its loop and a fifth of a launch
-// boundary), 10,000 4.1 -> 2.4, 200,000 25.8 -> 18.8, 10^6 118 -> 80.
+// boundary), 10,000 4.0 -> 2.4, 200,000 24.5 -> 17.6, 10^6 114 -> 76 (few spikes arriving).
 //
 // Spike lists: list 3 is the arena's, by step (the launches of one step);
 // 0..2 are span headers i % 3 with the records in span list i & 1.  A chunk of
@@ -240,7 +240,7 @@ struct Span {
     int kprev;       // first step of the launch before (its spikes are pushed now)
     int i;           // launch index in the chunk (span chunks)
     int src, dst;    // spike lists pushed from and appended to
-    int clear;       // span header this launch clears (-1: none; arena rotation for dst 3)
+    int clear;       // span header this launch clears (-1: none)
     int clear_arena; // clears the arena headers (the launch before the chunk's last)
 };
 

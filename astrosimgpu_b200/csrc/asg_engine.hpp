@@ -139,7 +139,8 @@ struct EngineConfig {
     int device = 0;
     int chunk_steps = 32;
     int block = 128;
-    int use_graphs = 1;  // 1 graphs of per-step launches, -1 plain launches, 2 persistent
+    int use_graphs = 1;  // 1 graphs of launches (of several steps where the delays allow),
+                         // -1 plain launches of one step, 2 persistent
     int sic_mode = 0;  // 0 auto, 1 fused, 2 split
     bool pdl = true;   // programmatic dependent launch between steps
     int push_mode = 0; // 0 deferred push when delays allow, 1 always in the spiking block

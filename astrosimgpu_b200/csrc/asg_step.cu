@@ -1655,9 +1655,7 @@ __global__ void __launch_bounds__(kMaxBlock) chunk_kernel(const InstDev* __restr
 // Side-stream SIC batch: a thread per target and arrival step (blockIdx.y) of
 // the batch sums the target's whole list (P = 1), the SIC role's sequential sum:
 // the factors of kSicBatch entries and the entries after them are loaded
-// together, then each entry's factor is added m times (a zero factor adds
-// +0.0, exact since a sum that starts at +0.0 and adds nonzero values is never
-// -0.0).
+// together, then each entry's factor is added m times, a zero factor none.
 // Launched when the step before step0+k has completed (the factors it
 // needs are older still), and waited for before the first step that reads it:
 // a batch that takes longer than the launches beside it is what the steps wait

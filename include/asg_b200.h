@@ -163,7 +163,9 @@ typedef struct asg_engine_opts {
                                <= 160 SIC edges per target, for a network (or a
                                batch) of >= 2^16 neurons; otherwise side-stream
                                batches when the delay is >= 12 steps, else the
-                               own role.                                        */
+                               own role.  Launches of several steps have no own
+                               role: the neuron's thread forms the current a step
+                               ahead there.                                     */
     int32_t pdl;            /* 0 = programmatic dependent launch (default), -1 off */
     int32_t push_mode;      /* 0 = spikes pushed one step later by load-balanced
                                push blocks when both spike delays are >= 2 steps
@@ -172,10 +174,11 @@ typedef struct asg_engine_opts {
                                buffers of launches of several steps; without room
                                for the latter one step per launch (0 = 90% free) */
     int32_t occupancy;      /* step kernel form: 0 auto (by the number of blocks
-                               a step launches), 1 latency form (fewest round
-                               trips, 128 registers), 2 high-occupancy form
-                               (6 blocks of 128 threads per SM; block 128 only).
-                               Both forms give the same bits.                  */
+                               a launch has), 1 latency form (fewest round
+                               trips; 4 blocks of 128 threads per SM, 3 in
+                               launches of several steps), 2 high-occupancy form
+                               (6, and 4; block 128 only).  All forms give the
+                               same bits.                                      */
     int32_t astro_precision;/* 0 or 64: FP64 (the product); 32: the astrocyte
                                update in FP32 -- the reference's precision
                                study (docs/experiments.md), opt-in, not
